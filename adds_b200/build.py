@@ -30,7 +30,7 @@ NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC",
                      "-Xcompiler", "-Wall", "-I", os.path.join(ROOT, "include")]
-CU_SOURCES = ["engine.cu", "phase.cu", "api.cu", "gen.cu", "adjoint.cu", "noalloc.cu", "diag.cu"]
+CU_SOURCES = ["engine.cu", "phase.cu", "wave.cu", "api.cu", "gen.cu", "adjoint.cu", "noalloc.cu", "diag.cu"]
 CXX_SOURCES = ["grio.cpp"]
 
 
@@ -56,6 +56,7 @@ def build(force: bool = False, verbose: bool = False, extra_nvcc=None) -> str:
     os.makedirs(LIBDIR, exist_ok=True)
     os.makedirs(BINDIR, exist_ok=True)
     headers = [os.path.join(CSRC, "adds_internal.h"), os.path.join(CSRC, "phase_internal.h"),
+               os.path.join(CSRC, "wave_internal.h"),
                os.path.join(ROOT, "include", "adds.h")]
     jobs = []
     objs = []

@@ -28,6 +28,7 @@
 #include "../../include/adds.h"
 #include "adds_internal.h"
 #include "phase_internal.h"
+#include "wave_internal.h"
 
 /* engine.cu */
 cudaError_t adds_engine_prepare(bool flt, int block, int *max_blocks_per_sm);
@@ -269,6 +270,7 @@ struct Knobs {
       light_heavy, block, greed;
   int engine, variant, group_ctas, solo_max, near_far, dense_scan; /* phase engine */
   int pull; /* phase engine: heavy phases may run as a pull (in-edge CSR)     */
+  int wave; /* wave kernel variant (WV_*) that solves instead of an engine, or -1 */
   unsigned long long timeout_ns;
 };
 
@@ -410,9 +412,15 @@ struct adds_graph {
   size_t bytes = 0;
   Engine eng;
   PhEngine peng;       /* phase engine (allocated on first use)            */
+  WvEngine weng;       /* wave kernels (allocated on first use)            */
+  bool wave_off = false; /* their lists overflowed on this graph           */
+  unsigned *wfirst = nullptr; /* pieces of long rows (WvQuery)              */
+  uint4 *wpiece = nullptr;
   unsigned trace_cap = 0; /* phase trace records requested (0 = off)       */
   PhParams last_pp;
   int last_engine = 0; /* engine of the solves in flight                   */
+  bool last_wave = false; /* ... which the wave kernels run                */
+  int last_shift = 0;     /* ... with this bucket shift                    */
   unsigned grow = 1;
   int tuned = 0;
   adds_opts tuned_opts;
@@ -564,6 +572,7 @@ extern "C" void adds_graph_free(adds_graph *g) {
   if (g->stream) cudaStreamSynchronize(g->stream);
   engine_free(g->eng);
   ph_engine_free(g->peng);
+  wv_engine_free(g->weng);
   if (g->row) cudaFree(g->row);
   if (g->edges) cudaFree(g->edges);
   if (g->dist) cudaFree(g->dist);
@@ -571,6 +580,8 @@ extern "C" void adds_graph_free(adds_graph *g) {
   if (g->split) cudaFree(g->split);
   if (g->trow) cudaFree(g->trow);
   if (g->tedges) cudaFree(g->tedges);
+  if (g->wfirst) cudaFree(g->wfirst);
+  if (g->wpiece) cudaFree(g->wpiece);
   if (g->aux) cudaFree(g->aux);
   if (g->sort_buf) cudaFree(g->sort_buf);
   if (g->sort_tmp) cudaFree(g->sort_tmp);
@@ -1044,6 +1055,18 @@ static void resolve(const adds_graph *g, const adds_opts *o, Knobs *k, int *shif
   k->pull = o->pull != 0 ? (o->pull > 0 ? 1 : 0) : (t->pull != 0 ? (t->pull > 0 ? 1 : 0) : 2);
   const int tmo = o->timeout_ms > 0 ? o->timeout_ms : 20000;
   k->timeout_ns = (unsigned long long)tmo * 1000000ull;
+  k->wave = o->wave > 0 ? std::min(o->wave - 1, WV_LAST) : -1;
+}
+
+/* True when the caller leaves the choice of engine and schedule to the
+ * library: only then may a solve go to the wave kernels by itself. */
+static bool schedule_auto(const adds_opts *o) {
+  return !o || (o->engine <= 0 && o->wave == 0 && o->delta_shift < 0 && o->delta_scale <= 0.f &&
+                o->window <= 0 && o->ctas_per_sm <= 0 && o->batch_max <= 0 &&
+                o->hub_threshold <= 0 && o->adapt < 0 && o->strict_order < 0 &&
+                o->local_max < 0 && o->light_heavy < 0 && o->block_threads <= 0 &&
+                o->greed < 0 && o->group_ctas <= 0 && o->solo_max < 0 && o->near_far <= 0 &&
+                o->dense_scan == 0 && o->pull == 0);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -1315,6 +1338,93 @@ static int graph_phase_engine(adds_graph *g, const Knobs &k, int shift, float sc
   return rc;
 }
 
+/* Pieces of the rows that one warp of a wave kernel should not relax alone:
+ * counted per row, numbered by a scan, written out.  Depends on the rows
+ * only, so it is made once per graph. */
+__global__ void k_piece_count(const unsigned *row, uint32_t n, unsigned *cnt) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x) {
+    const unsigned deg = v < n ? row[v + 1] - row[v] : 0u;
+    cnt[v] = deg > WV_PIECE ? (deg + WV_PIECE - 1u) / WV_PIECE : 0u;
+  }
+}
+__global__ void k_piece_fill(const unsigned *row, uint32_t n, const unsigned *first, uint4 *piece) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const unsigned r1 = row[v + 1], c1 = first[v + 1];
+    unsigned e = row[v];
+    for (unsigned c = first[v]; c < c1; ++c, e += WV_PIECE)
+      piece[c] = make_uint4(v, e, min(WV_PIECE, r1 - e), 0u);
+  }
+}
+
+static int graph_pieces(adds_graph *g) {
+  if (g->wpiece || g->max_deg <= WV_PIECE) return ADDS_OK;
+  const size_t n = g->n;
+  unsigned *cnt = nullptr;
+  void *tmp = nullptr;
+  size_t tb = 0;
+  unsigned total = 0;
+  cudaError_t e = cudaSuccess;
+  if (!g->wfirst) e = cudaMalloc(&g->wfirst, (n + 1) * 4);
+  if (e == cudaSuccess) e = cudaMalloc(&cnt, (n + 1) * 4);
+  if (e == cudaSuccess) {
+    k_piece_count<<<592, 256, 0, g->stream>>>(g->row, g->n, cnt);
+    e = cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, g->wfirst, (int)(n + 1), g->stream);
+  }
+  if (e == cudaSuccess) e = cudaMalloc(&tmp, tb ? tb : 16);
+  if (e == cudaSuccess)
+    e = cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, g->wfirst, (int)(n + 1), g->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&total, g->wfirst + n, 4, cudaMemcpyDeviceToHost, g->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+  if (e == cudaSuccess) e = cudaMalloc(&g->wpiece, ((size_t)total + 1) * sizeof(uint4));
+  if (e == cudaSuccess) {
+    k_piece_fill<<<592, 256, 0, g->stream>>>(g->row, g->n, g->wfirst, g->wpiece);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+  if (cnt) cudaFree(cnt);
+  if (tmp) cudaFree(tmp);
+  if (e != cudaSuccess) {
+    if (g->wpiece) cudaFree(g->wpiece);
+    g->wpiece = nullptr;
+    return cuda_fail(e, "pieces of long rows");
+  }
+  g->bytes += (n + 1) * 4 + (size_t)total * sizeof(uint4);
+  return ADDS_OK;
+}
+
+/* first threshold step of the wave kernels, in distance units */
+static float wave_delta(const adds_graph *g, int shift, float scale) {
+  const double d = ldexp(1.0, shift);
+  return (float)(g->wt == ADDS_F32 ? d / (double)scale : d);
+}
+
+static int graph_wave_engine(adds_graph *g, const Knobs &k, int shift, float scale) {
+  const int rp = graph_pieces(g);
+  if (rp) return rp;
+  WvQuery q;
+  memset(&q, 0, sizeof q);
+  q.row = g->row;
+  q.edges = g->edges;
+  q.first = g->wfirst;
+  q.piece = g->wpiece;
+  q.dist = g->dist;
+  q.n = g->n;
+  q.m = g->m;
+  q.delta = wave_delta(g, shift, scale);
+  WvEngine &E = g->weng;
+  const unsigned gs = (unsigned)std::max(0, k.group_ctas);
+  if (E.nq == 1 && E.shape == k.wave && E.req_gsize == gs) {
+    if (E.qs_host[0].delta == q.delta) return ADDS_OK;
+    E.qs_host[0] = q;
+    return wv_engine_upload(E, g->stream) ? ADDS_ERR_CUDA : ADDS_OK;
+  }
+  const int rc = wv_engine_alloc(E, g->device, g->wt == ADDS_F32, k.wave, gs,
+                                 std::vector<WvQuery>(1, q), g->stream);
+  if (rc) snprintf(g_last_err, sizeof g_last_err, "wave kernel allocation failed (%d)", rc);
+  return rc;
+}
+
 extern "C" int adds_graph_trace(adds_graph *g, uint32_t cap) {
   if (!g || cap > (1u << 24)) return ADDS_ERR_INVALID;
   int rc = set_device(g->device);
@@ -1363,8 +1473,81 @@ static void fill_phase_stats(const PhEngine &E, adds_stats *s) {
   s->repushes = g.st_repush;
 }
 
+static void fill_wave_stats(const WvEngine &E, adds_stats *s) {
+  if (!s) return;
+  const WvStat &t = *E.st_host;
+  s->items_popped = t.items;
+  s->items_stale = t.stale;
+  s->edges_scanned = t.edges;
+  s->pushes = t.pushes;
+  s->phases = t.steps;
+  s->batches = t.splits;
+  s->ctas = (int32_t)E.ctas;
+  s->launches = 1;
+}
+
+/* error word, reset and counters of whatever ran g's last solves */
+static int graph_status(const adds_graph *g) {
+  if (g->last_wave) return wv_engine_status(g->weng, g_last_err, sizeof g_last_err);
+  return g->last_engine == ADDS_ENGINE_PHASE ? phase_status(g->peng) : engine_status(g->eng);
+}
+static void graph_reset(adds_graph *g, cudaStream_t st) {
+  if (g->last_wave) wv_engine_reset(g->weng, st);
+  else if (g->last_engine == ADDS_ENGINE_PHASE) ph_engine_reset(g->peng, st);
+  else engine_full_reset(g->eng, st);
+}
+/* after a worklist overflow: a larger pool on the rerun, or, for the wave
+ * kernels, whose lists are sized once, the engine that has one */
+static void graph_outgrown(adds_graph *g) {
+  if (g->last_wave) {
+    g->wave_off = true;
+    wv_engine_free(g->weng);
+    return;
+  }
+  g->grow *= 2;
+  if (g->last_engine == ADDS_ENGINE_PHASE) ph_engine_free(g->peng); else engine_free(g->eng);
+}
+static void graph_stats(const adds_graph *g, adds_stats *stats, double ms, double kms) {
+  if (!stats) return;
+  memset(stats, 0, sizeof *stats);
+  stats->ms = ms;
+  stats->kernel_ms = kms;
+  if (g->last_wave) {
+    fill_wave_stats(g->weng, stats);
+    stats->engine = g->last_engine;
+    stats->delta_shift = g->last_shift;
+  } else if (g->last_engine == ADDS_ENGINE_PHASE) {
+    fill_phase_stats(g->peng, stats);
+    stats->delta_shift = (int32_t)g->peng.qs_host[0].shift;
+  } else {
+    fill_stats(g->eng, g->last_params, stats);
+    stats->delta_shift = (int32_t)g->eng.qs_host[0].shift0;
+    stats->engine = ADDS_ENGINE_ASYNC;
+  }
+}
+
 static cudaStream_t pick_stream(const adds_graph *g, const adds_opts *o) {
   return (o && o->stream) ? (cudaStream_t)o->stream : g->stream;
+}
+
+/* The wave kernel of a plain solve whose schedule is left to the library, or
+ * none.  Measured on one B200, untuned solves with automatic knobs (wave
+ * kernel against the phase engine, which they ran on before; the asynchronous
+ * engine in brackets):
+ *   average degree under 6: 64^2 grid 0.25 against 2.2 ms (0.58), 300^2 0.88
+ *   against 14.9 (1.8), 4096^2 18.3 against 310 (38); one CTA below 4,096
+ *   vertices, where a group's exchanges cost what its width saves (16^2 0.107
+ *   against 0.118, 64^2 0.295 against 0.25);
+ *   longer rows: ER 4,001 x 8 0.16 against 0.57 (0.29), ER 10^6 x 8 0.6 against
+ *   1.8 (0.95), R-MAT 16 0.38 against 0.87 (0.49), R-MAT 20 1.3 against 1.8
+ *   (1.15).  The wave kernel relaxes whole rows (3 to 5 times each edge of an
+ *   R-MAT graph), so from 2^25 edges on the phase engine's light/heavy split
+ *   and pull phases win. */
+static int auto_wave(const adds_graph *g, const adds_opts *o) {
+  if (g->wave_off || g->trace_cap || !schedule_auto(o)) return -1;
+  if (g->tuned) return g->tuned_opts.wave > 0 ? g->tuned_opts.wave - 1 : -1;
+  if (g->avg_deg < 6.0 && g->m < (1ull << 31)) return g->n < 4096u ? WV_WIDE : WV_GROUP;
+  return g->m < (1ull << 25) ? WV_POOL : -1;
 }
 
 /* Enqueues one solve; no host synchronisation.  Each solve records four
@@ -1374,12 +1557,25 @@ static int sssp_enqueue(adds_graph *g, uint32_t src, const adds_opts *opts) {
   float scale;
   Knobs k;
   resolve(g, opts, &k, &shift, &scale);
-  const bool phase = k.engine == ADDS_ENGINE_PHASE;
-  int rc = phase ? graph_phase_engine(g, k, shift, scale) : graph_engine(g, k, shift, scale);
+  if (k.wave < 0) k.wave = auto_wave(g, opts);
+  if (g->wave_off) k.wave = -1;
+  const bool phase = k.engine == ADDS_ENGINE_PHASE, wave = k.wave >= 0;
+  int rc = ADDS_OK;
+  if (wave) {
+    rc = graph_wave_engine(g, k, shift, scale);
+    if (rc == ADDS_ERR_OOM || rc == ADDS_ERR_UNSUPPORTED) { /* no room for its lists */
+      g->wave_off = true;
+      return sssp_enqueue(g, src, opts);
+    }
+  } else {
+    rc = phase ? graph_phase_engine(g, k, shift, scale) : graph_engine(g, k, shift, scale);
+  }
   if (rc) return rc;
   cudaStream_t st = pick_stream(g, opts);
   g->last_knobs = k;
   g->last_engine = k.engine;
+  g->last_wave = wave;
+  g->last_shift = shift;
   if (g->ring_used == adds_graph::kRing) { /* ring full: fold into nothing */
     CK(cudaStreamSynchronize(st));
     g->ring_used = 0;
@@ -1388,7 +1584,10 @@ static int sssp_enqueue(adds_graph *g, uint32_t src, const adds_opts *opts) {
   for (int j = 0; j < 4; ++j)
     if (!ev[j]) CK(cudaEventCreate(&ev[j]));
   CK(cudaEventRecord(ev[0], st));
-  if (phase) {
+  if (wave) {
+    if (wv_engine_enqueue(g->weng, src, k.timeout_ns, st, ev[1], ev[2]))
+      return cuda_fail(cudaGetLastError(), "wave kernel launch");
+  } else if (phase) {
     PhParams P;
     if (ph_engine_params(g->peng, phase_knobs(k), src, &P)) return ADDS_ERR_INVALID;
     g->last_pp = P;
@@ -1435,18 +1634,15 @@ extern "C" int adds_sssp(adds_graph *g, uint32_t src, void *dist_out, const adds
     rc = sssp_enqueue(g, src, opts);
     if (rc) return rc;
     CK(cudaStreamSynchronize(st));
-    const bool phase = g->last_engine == ADDS_ENGINE_PHASE;
-    rc = phase ? phase_status(g->peng) : engine_status(g->eng);
+    rc = graph_status(g);
     if (rc == ADDS_ERR_WL_OVERFLOW && retries < 4) {
       ++retries;
-      g->grow *= 2;
-      /* re-allocated at the larger size on the rerun */
-      if (phase) ph_engine_free(g->peng); else engine_free(g->eng);
+      graph_outgrown(g); /* re-allocated at the larger size on the rerun */
       g->ring_used = 0;
       continue;
     }
     if (rc) {
-      if (phase) ph_engine_reset(g->peng, st); else engine_full_reset(g->eng, st);
+      graph_reset(g, st);
       g->ring_used = 0;
       return rc;
     }
@@ -1454,20 +1650,8 @@ extern "C" int adds_sssp(adds_graph *g, uint32_t src, void *dist_out, const adds
   }
   double ms = 0, kms = 0;
   ring_times(g, &ms, &kms);
-  if (stats) {
-    memset(stats, 0, sizeof *stats);
-    stats->ms = ms;
-    stats->kernel_ms = kms;
-    if (g->last_engine == ADDS_ENGINE_PHASE) {
-      fill_phase_stats(g->peng, stats);
-      stats->delta_shift = (int32_t)g->peng.qs_host[0].shift;
-    } else {
-      fill_stats(g->eng, g->last_params, stats);
-      stats->delta_shift = (int32_t)g->eng.qs_host[0].shift0;
-      stats->engine = ADDS_ENGINE_ASYNC;
-    }
-    stats->retries = retries;
-  }
+  graph_stats(g, stats, ms, kms);
+  if (stats) stats->retries = retries;
   g->pending = 0;
   if (dist_out) return adds_graph_last_dist(g, dist_out);
   return ADDS_OK;
@@ -1544,12 +1728,11 @@ extern "C" int adds_sssp_sources(adds_graph *g, const uint32_t *srcs, uint32_t n
   }
   if (e1 != cudaSuccess || e2 != cudaSuccess)
     return cuda_fail(e1 != cudaSuccess ? e1 : e2, "multi-source solve");
-  const bool phase = g->last_engine == ADDS_ENGINE_PHASE;
-  rc = phase ? phase_status(g->peng) : engine_status(g->eng);
+  rc = graph_status(g);
   if (rc == ADDS_ERR_WL_OVERFLOW) {
     /* the worklist outgrew its pool: solve one at a time, which regrows it */
     g->ring_used = 0;
-    if (phase) ph_engine_reset(g->peng, st); else engine_full_reset(g->eng, st);
+    graph_reset(g, st);
     for (uint32_t i = 0; i < ns; ++i) {
       rc = adds_sssp(g, srcs[i], dist_out[i], opts, i + 1 == ns ? stats : nullptr);
       if (rc) return rc;
@@ -1557,25 +1740,13 @@ extern "C" int adds_sssp_sources(adds_graph *g, const uint32_t *srcs, uint32_t n
     return ADDS_OK;
   }
   if (rc) {
-    if (phase) ph_engine_reset(g->peng, st); else engine_full_reset(g->eng, st);
+    graph_reset(g, st);
     g->ring_used = 0;
     return rc;
   }
   double ms = 0, kms = 0;
   ring_times(g, &ms, &kms);
-  if (stats) {
-    memset(stats, 0, sizeof *stats);
-    stats->ms = ms;
-    stats->kernel_ms = kms;
-    if (phase) {
-      fill_phase_stats(g->peng, stats);
-      stats->delta_shift = (int32_t)g->peng.qs_host[0].shift;
-    } else {
-      fill_stats(g->eng, g->last_params, stats);
-      stats->delta_shift = (int32_t)g->eng.qs_host[0].shift0;
-      stats->engine = ADDS_ENGINE_ASYNC;
-    }
-  }
+  graph_stats(g, stats, ms, kms);
   g->pending = 0;
   return ADDS_OK;
 }
@@ -1604,8 +1775,8 @@ extern "C" int adds_graph_sync(adds_graph *g, adds_stats *stats) {
   double ms = 0, kms = 0;
   ring_times(g, &ms, &kms);
   const bool phase = g->last_engine == ADDS_ENGINE_PHASE;
-  if (phase ? g->peng.nq == 0 : g->eng.nq == 0) return ADDS_OK;
-  rc = phase ? phase_status(g->peng) : engine_status(g->eng);
+  if (g->last_wave ? g->weng.nq == 0 : phase ? g->peng.nq == 0 : g->eng.nq == 0) return ADDS_OK;
+  rc = graph_status(g);
   g->pending = 0;
   std::vector<std::pair<uint32_t, adds_opts>> redo;
   redo.swap(g->pend);
@@ -1613,8 +1784,7 @@ extern "C" int adds_graph_sync(adds_graph *g, adds_stats *stats) {
     /* a solve outgrew the worklist pool (and the ones after it exited):
      * run them all again one at a time, as adds_sssp does, on a larger pool;
      * the graph then holds the last one's distances as it would have */
-    if (phase) ph_engine_free(g->peng); else engine_free(g->eng);
-    g->grow *= 2;
+    graph_outgrown(g);
     for (size_t i = 0; i < redo.size(); ++i) {
       rc = adds_sssp(g, redo[i].first, nullptr, &redo[i].second,
                      i + 1 == redo.size() ? stats : nullptr);
@@ -1623,22 +1793,10 @@ extern "C" int adds_graph_sync(adds_graph *g, adds_stats *stats) {
     return ADDS_OK;
   }
   if (rc) {
-    if (phase) ph_engine_reset(g->peng, g->stream); else engine_full_reset(g->eng, g->stream);
+    graph_reset(g, g->stream);
     return rc;
   }
-  if (stats) {
-    memset(stats, 0, sizeof *stats);
-    stats->ms = ms;
-    stats->kernel_ms = kms;
-    if (phase) {
-      fill_phase_stats(g->peng, stats);
-      stats->delta_shift = (int32_t)g->peng.qs_host[0].shift;
-    } else {
-      fill_stats(g->eng, g->last_params, stats);
-      stats->delta_shift = (int32_t)g->eng.qs_host[0].shift0;
-      stats->engine = ADDS_ENGINE_ASYNC;
-    }
-  }
+  graph_stats(g, stats, ms, kms);
   return ADDS_OK;
 }
 
@@ -1684,6 +1842,7 @@ struct adds_batch {
   std::vector<size_t> dist_off;
   Engine eng;
   PhEngine peng; /* used when kn.engine is ADDS_ENGINE_PHASE */
+  WvEngine weng; /* used when kn.wave names a variant */
   PhParams pp;
   unsigned grow = 1;
   Knobs kn;
@@ -1740,9 +1899,43 @@ static int batch_phase_engine(adds_batch *b) {
   return ADDS_OK;
 }
 
+static int batch_wave_engine(adds_batch *b) {
+  std::vector<WvQuery> qv(b->qgraph.size());
+  for (size_t i = 0; i < qv.size(); ++i) {
+    adds_graph *g = b->qgraph[i];
+    const int rp = graph_pieces(g);
+    if (rp) return rp;
+    WvQuery q;
+    memset(&q, 0, sizeof q);
+    q.row = g->row;
+    q.edges = g->edges;
+    q.first = g->wfirst;
+    q.piece = g->wpiece;
+    q.dist = b->dist_all + b->dist_off[i];
+    q.n = g->n;
+    q.m = g->m;
+    q.src = b->srcs[i];
+    q.delta = wave_delta(g, b->shifts[i], b->scales[i]);
+    qv[i] = q;
+  }
+  if (b->exec) {
+    cudaGraphExecDestroy(b->exec);
+    b->exec = nullptr;
+  }
+  b->captured = false;
+  const int rc = wv_engine_alloc(b->weng, b->device, b->flt, b->kn.wave, 0u, qv, b->stream);
+  if (rc) snprintf(g_last_err, sizeof g_last_err, "wave kernel allocation failed (%d)", rc);
+  return rc;
+}
+
 static int batch_engine(adds_batch *b) {
   b->wversions.clear();
   for (adds_graph *g : b->ugraph) b->wversions.push_back(g->wversion);
+  if (b->kn.wave >= 0) {
+    const int rw = batch_wave_engine(b);
+    if (rw != ADDS_ERR_OOM && rw != ADDS_ERR_UNSUPPORTED) return rw;
+    b->kn.wave = -1; /* no room for its lists */
+  }
   if (b->kn.engine == ADDS_ENGINE_PHASE) return batch_phase_engine(b);
   std::vector<EngQuery> qv(b->qgraph.size());
   for (size_t i = 0; i < qv.size(); ++i) {
@@ -1832,6 +2025,15 @@ extern "C" int adds_batch_create(adds_graph *const *graphs, const uint32_t *srcs
     int s_unused;
     float sc_unused;
     resolve(graphs[big], &lw, &b->kn, &s_unused, &sc_unused, false);
+    /* Sparse graphs with the schedule left to the library: one CTA per query
+     * on the wave kernels.  128 grids x 16 sources 7.3 ms against 98 on the
+     * asynchronous engine; 60 sources on a 257 x 255 road 1.6 against 4.7
+     * (1,024 threads a query while every query has an SM to itself: 2.4 ms
+     * with 256). */
+    bool sparse = schedule_auto(opts);
+    for (adds_graph *g : b->ugraph) sparse = sparse && g->avg_deg < 6.0 && g->m < (1ull << 31);
+    if (sparse) b->kn.wave = nq <= 148u ? WV_WIDE : WV_CTA;
+    if (b->kn.wave >= WV_GROUP && nq != 1u) b->kn.wave = WV_WIDE; /* groups solve one query */
   }
   /* the batch sizes its groups itself unless the caller says otherwise */
   b->kn.group_ctas = (opts && opts->group_ctas > 0) ? opts->group_ctas : 0;
@@ -1858,6 +2060,7 @@ extern "C" void adds_batch_free(adds_batch *b) {
   if (b->exec) cudaGraphExecDestroy(b->exec);
   engine_free(b->eng);
   ph_engine_free(b->peng);
+  wv_engine_free(b->weng);
   if (b->dist_all) cudaFree(b->dist_all);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
@@ -1869,10 +2072,24 @@ extern "C" void adds_batch_free(adds_batch *b) {
 }
 
 /* init + solve + status read-back, captured once as a CUDA graph */
+static int batch_status(const adds_batch *b) {
+  if (b->kn.wave >= 0) return wv_engine_status(b->weng, g_last_err, sizeof g_last_err);
+  return b->kn.engine == ADDS_ENGINE_PHASE ? phase_status(b->peng) : engine_status(b->eng);
+}
+static void batch_reset(adds_batch *b) {
+  if (b->kn.wave >= 0) wv_engine_reset(b->weng, b->stream);
+  else if (b->kn.engine == ADDS_ENGINE_PHASE) ph_engine_reset(b->peng, b->stream);
+  else engine_full_reset(b->eng, b->stream);
+}
+
 static int batch_capture(adds_batch *b) {
   cudaGraph_t gr = nullptr;
   CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = b->kn.engine == ADDS_ENGINE_PHASE
+  int rc = b->kn.wave >= 0
+               ? (wv_engine_enqueue(b->weng, 0xFFFFFFFFu, b->kn.timeout_ns, b->stream, b->k0, b->k1)
+                      ? ADDS_ERR_CUDA
+                      : ADDS_OK)
+           : b->kn.engine == ADDS_ENGINE_PHASE
                ? (ph_engine_enqueue(b->peng, b->pp, b->stream, b->k0, b->k1) ? ADDS_ERR_CUDA : ADDS_OK)
                : engine_enqueue(b->eng, b->P, b->stream, b->k0, b->k1);
   cudaError_t e = cudaStreamEndCapture(b->stream, &gr);
@@ -1895,6 +2112,10 @@ static int batch_relayout(adds_batch *b) {
   for (size_t i = 0; i < b->ugraph.size(); ++i)
     if (b->ugraph[i]->wversion != b->wversions[i]) changed = true;
   if (!changed) return ADDS_OK;
+  if (b->kn.wave >= 0) { /* the CSR itself, whose weights changed in place */
+    for (size_t i = 0; i < b->ugraph.size(); ++i) b->wversions[i] = b->ugraph[i]->wversion;
+    return ADDS_OK;
+  }
   for (size_t i = 0; i < b->qgraph.size(); ++i) {
     const uint2 *edges;
     const unsigned *split;
@@ -1939,10 +2160,9 @@ extern "C" int adds_batch_sync(adds_batch *b, adds_stats *stats) {
   CK(cudaSetDevice(b->device));
   CK(cudaStreamSynchronize(b->stream));
   const bool phase = b->kn.engine == ADDS_ENGINE_PHASE;
-  int rc = phase ? phase_status(b->peng) : engine_status(b->eng);
+  int rc = batch_status(b);
   if (rc) {
-    /* reported: the next launch starts from a clean engine */
-    if (phase) ph_engine_reset(b->peng, b->stream); else engine_full_reset(b->eng, b->stream);
+    batch_reset(b); /* reported: the next launch starts from a clean engine */
     return rc;
   }
   if (stats) {
@@ -1952,7 +2172,10 @@ extern "C" int adds_batch_sync(adds_batch *b, adds_stats *stats) {
     CK(cudaEventElapsedTime(&kms, b->k0, b->k1));
     stats->ms = ms;
     stats->kernel_ms = kms;
-    if (phase) {
+    if (b->kn.wave >= 0) {
+      fill_wave_stats(b->weng, stats);
+      stats->engine = b->kn.engine;
+    } else if (phase) {
       fill_phase_stats(b->peng, stats);
     } else {
       fill_stats(b->eng, b->P, stats);
@@ -1972,14 +2195,18 @@ extern "C" int adds_batch_run(adds_batch *b, adds_stats *stats) {
     rc = adds_batch_sync(b, stats);
     if (rc == ADDS_ERR_WL_OVERFLOW && retries < 4) {
       ++retries;
-      b->grow *= 2;
+      if (b->kn.wave >= 0) { /* its lists do not grow: the engine that does */
+        wv_engine_free(b->weng);
+        b->kn.wave = -1;
+      } else {
+        b->grow *= 2;
+      }
       rc = batch_engine(b);
       if (rc) return rc;
       continue;
     }
     if (rc) {
-      if (b->kn.engine == ADDS_ENGINE_PHASE) ph_engine_reset(b->peng, b->stream);
-      else engine_full_reset(b->eng, b->stream);
+      batch_reset(b);
       return rc;
     }
     if (stats) stats->retries = retries;
@@ -1994,6 +2221,10 @@ extern "C" int adds_batch_set_sources(adds_batch *b, const uint32_t *srcs) {
   CK(cudaSetDevice(b->device));
   CK(cudaStreamSynchronize(b->stream));
   for (size_t i = 0; i < b->srcs.size(); ++i) b->srcs[i] = srcs[i];
+  if (b->kn.wave >= 0) {
+    for (size_t i = 0; i < b->srcs.size(); ++i) b->weng.qs_host[i].src = srcs[i];
+    return wv_engine_upload(b->weng, b->stream) ? ADDS_ERR_CUDA : ADDS_OK;
+  }
   if (b->kn.engine == ADDS_ENGINE_PHASE) {
     for (size_t i = 0; i < b->srcs.size(); ++i) b->peng.qs_host[i].src = srcs[i];
     return ph_engine_upload(b->peng, b->stream) ? ADDS_ERR_CUDA : ADDS_OK;
@@ -2248,6 +2479,22 @@ extern "C" int adds_tune(adds_graph *g, const uint32_t *srcs, uint32_t ns, adds_
     bm = descend(cur, bm, &cur);
   }
   if (bm >= 1e29) return ADDS_ERR_DEVICE_TIMEOUT;
+  if (want == ADDS_ENGINE_AUTO && g->m < (1ull << 31)) {
+    /* the wave kernels, on the heuristic's width (they adapt it) */
+    adds_opts w;
+    adds_opts_init(&w);
+    w.engine = cur.engine;
+    for (int v = 0; v <= WV_LAST; ++v) {
+      g->wave_off = false;
+      w.wave = v + 1;
+      const double ms = time_solves(g, srcs, ns, &w);
+      if (!g->wave_off && ms < bm * 0.98) { /* off: its lists overflowed */
+        bm = ms;
+        cur.wave = v + 1;
+      }
+    }
+    g->wave_off = false;
+  }
   g->tuned_opts = cur;
   g->tuned_opts.stream = nullptr;
   g->tuned = 1;

@@ -1,0 +1,1028 @@
+/*
+ * wave.cu — near-far SSSP by one CTA or one thread-block cluster per query.
+ *
+ * Replaces, for thin wave fronts and for batches of many queries, the
+ * worklist of the reference (ads_int/wl.h:133-1972) and its relaxation
+ * (ads_int/kernel.cu:30-128).  A road network's wave front is a chain of a
+ * thousand or more dependent steps; what a step costs is its memory round
+ * trips and its barrier, not its bytes.  Here a group that can synchronise in
+ * hardware (a CTA, or a cluster of CTAs) runs the chain alone: the frontier
+ * lives in shared memory, the step's barrier is bar.sync or
+ * barrier.cluster, and nothing is counted, published or claimed through HBM.
+ * Many groups run side by side (a batch), one after another from a shared
+ * counter, largest first.
+ *
+ * A step pops the frontier's entries (v, d), drops those that a smaller
+ * distance has superseded, relaxes the rows and keeps the improvements: those
+ * below the near threshold T are the next frontier, the others go to the
+ * CTA's far list.  When the frontier is empty, or small while far entries
+ * wait, T moves up and the far list is split again (stale entries dropped,
+ * the rest kept).  Any sequence of thresholds is label-correcting, so the
+ * distances are the fixed point that every other engine reaches.
+ *
+ * An improvement is pushed by the one thread whose atomicMin lowered the
+ * distance: steps are in lock step, so pushing on the gathered value alone
+ * (as the asynchronous engine does) would push a vertex once for each of its
+ * equal paths, and those copies multiply from step to step.
+ *
+ * What bounds it: the chain of memory round trips of a hop (row bounds, edges,
+ * atomicMin and its answer: about 3,400 cycles with the push and the barrier,
+ * in a group; a load from L2 takes 310 to 460 cycles, an atomic 510 to 870),
+ * and, where a CTA has hundreds of entries, its rate of scattered requests
+ * (one sector a cycle and SM, an atomic two cycles).  Hence: the row bounds of
+ * an improvement are prefetched while its atomicMin is on its way, four lanes
+ * share a vertex so that a row comes with one request, and small hops skip the
+ * filtering load of the distance before the atomic.  A group's CTAs run several
+ * hops on their own entries between two exchanges, which cost about 6,000
+ * cycles: neighbouring entries stay together, so few of these hops relax from a
+ * distance that another CTA is about to lower.
+ *
+ * Measured (one B200, automatic knobs, before -> now): 4096^2 road-like grid
+ * 261-310 -> 18.1 ms; 517 x 301 road 16-21 -> 0.85 ms; 128 grids x 16 sources in
+ * one batch 97.7 -> 7.2 ms; 60 sources on a 257 x 255 road 4.7 -> 1.6 ms; R-MAT 16
+ * 0.87 -> 0.37 ms; ER 4,001 x 8 0.57 -> 0.15 ms.
+ *
+ * The lists cannot grow: an overflow ends the launch with WV_ERR_OVERFLOW and
+ * the host solves on another engine.
+ */
+#include <cuda_runtime.h>
+#include <stddef.h>
+#include <stdio.h>
+#include <string.h>
+
+#include <algorithm>
+
+#include "../../include/adds.h"
+#include "adds_internal.h"
+#include "wave_internal.h"
+
+namespace adds_wave {
+
+__device__ __forceinline__ unsigned long long gtimer() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+/* what the CTAs of a group tell each other at an exchange */
+struct __align__(16) Note {
+  unsigned near_cnt, far_cnt, far_min, stop;
+};
+
+/* a hop's pushes: entries of the next frontier, far entries added, error.
+ * Three of them rotate: the one a hop reads, the one it fills, and the one it
+ * clears for the next, so that a hop needs one barrier. */
+struct __align__(16) Ctr {
+  unsigned near_cnt, far_new, stop;
+  unsigned cut; /* a long row became pieces */
+};
+
+template <int BLOCK, int NS, bool POOL>
+struct WSmem {
+  uint2 nb[2][NS];  /* frontier entries (v, d): this hop's, the next          */
+  Ctr ctr[3];
+  Note tot;         /* the group's totals                                     */
+  unsigned kept;    /* far entries a split has kept                           */
+  unsigned fmin;    /* the smallest distance among them                       */
+  unsigned q, r0;
+  unsigned pre[WV_MAX_GROUP]; /* inclusive frontier counts of the CTAs        */
+  /* POOL: the rows being relaxed by the whole CTA, and their edge offsets    */
+  static constexpr int PB = POOL ? BLOCK : 1;
+  unsigned it_r0[PB], it_d[PB], it_off[PB + 1], wsum[32];
+};
+
+/* lists of one CTA in HBM */
+struct Lists {
+  uint2 *over;      /* frontier entries past the shared ones: two areas       */
+  uint2 *far;
+  unsigned ncap, fcap;
+};
+
+template <bool FLT>
+__device__ __forceinline__ unsigned add_word(unsigned d, unsigned w) {
+  return FLT ? __float_as_uint(__fadd_rn(__uint_as_float(d), __uint_as_float(w))) : d + w;
+}
+
+/* threshold word of distance word d plus delta; never below d + 1, so that a
+ * threshold taken from an entry always admits it */
+template <bool FLT>
+__device__ __forceinline__ unsigned raise_word(unsigned d, float delta) {
+  unsigned t;
+  if (FLT) {
+    t = __float_as_uint(__fadd_rn(__uint_as_float(d), delta));
+  } else {
+    const double x = (double)d + (double)delta;
+    t = x < 4294967295.0 ? (unsigned)x : 0xFFFFFFFFu;
+  }
+  return t > d ? t : d + (d != 0xFFFFFFFFu);
+}
+
+/* a note in one 16-byte access */
+__device__ __forceinline__ void st_note(ulonglong2 *p, unsigned a, unsigned b, unsigned c,
+                                        unsigned d) {
+  const unsigned long long lo = a | ((unsigned long long)b << 32);
+  const unsigned long long hi = c | ((unsigned long long)d << 32);
+  asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p),
+               "l"(lo), "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ uint4 ld_note(const ulonglong2 *p) {
+  unsigned long long lo, hi;
+  asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  return make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
+}
+
+/* GRP: several CTAs per query.  POOL: a CTA pools the edges of its entries
+ * over all its threads (graphs whose rows differ much in length); without it
+ * each warp relaxes its own entries. */
+template <bool FLT, int BLOCK, int NS, bool GRP, bool POOL>
+struct Wave {
+  using Smem = WSmem<BLOCK, NS, POOL>;
+
+  /* one thread's state over a query; all but the counts is uniform */
+  struct State {
+    Lists L;
+    const unsigned *row;
+    const uint2 *edges;
+    const unsigned *first; /* long rows: a row's first piece, the pieces       */
+    const uint4 *piece;
+    unsigned *dist;
+    unsigned n;
+    unsigned T;    /* near threshold (distance word)                          */
+    unsigned cur;  /* frontier buffer being read                              */
+    unsigned ci;   /* counter of that frontier                                */
+    unsigned F;    /* far entries of this CTA                                 */
+    unsigned npush, nstale;
+    unsigned long long nedge;
+  };
+  static __device__ __forceinline__ unsigned next3(unsigned i) { return i == 2u ? 0u : i + 1u; }
+
+  static __device__ __forceinline__ uint2 entry(const Smem &S, const State &w, unsigned i) {
+    return i < NS ? S.nb[w.cur][i] : __ldcg(w.L.over + (size_t)w.cur * w.L.ncap + (i - NS));
+  }
+  static __device__ __forceinline__ void put(Smem &S, const State &w, unsigned buf, unsigned i,
+                                             uint2 e) {
+    if (i < NS) S.nb[buf][i] = e;
+    else if (i - NS < w.L.ncap) __stcg(w.L.over + (size_t)buf * w.L.ncap + (i - NS), e);
+  }
+
+  /* Relaxes the edges ed (those in msk) of each lane from distance words dd
+   * and pushes the improvements: one reservation per list and warp. */
+  template <int U>
+  static __device__ __forceinline__ void relax(Smem &S, State &w, const uint2 (&ed)[U],
+                                               const unsigned (&dd)[U], unsigned msk,
+                                               bool direct = false) {
+    const unsigned lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    unsigned nd[U], cur[U], bn[U], bf[U], cn = 0, cf = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      nd[u] = add_word<FLT>(dd[u], ed[u].y);
+      cur[u] = 0u;
+      if ((msk >> u) & 1u) cur[u] = direct ? 0xFFFFFFFFu : __ldcg(w.dist + ed[u].x);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) { /* absent edges hold cur 0: never below */
+      if (nd[u] < cur[u]) {
+        cur[u] = atomicMin(w.dist + ed[u].x, nd[u]);
+        /* the row bounds are wanted as soon as the entry is popped */
+        if (GRP && nd[u] < w.T)
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(w.row + ed[u].x));
+      } else {
+        cur[u] = 0u;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool p = nd[u] < cur[u], nr = nd[u] < w.T;
+      bn[u] = __ballot_sync(0xFFFFFFFFu, p && nr);
+      bf[u] = __ballot_sync(0xFFFFFFFFu, p && !nr);
+      cn += __popc(bn[u]);
+      cf += __popc(bf[u]);
+    }
+    if ((cn | cf) == 0u) return;
+    Ctr &C = S.ctr[next3(w.ci)];
+    unsigned at = 0;
+    if (lane < 2u) at = atomicAdd(lane ? &C.far_new : &C.near_cnt, lane ? cf : cn);
+    unsigned pn = __shfl_sync(0xFFFFFFFFu, at, 0);
+    unsigned pf = __shfl_sync(0xFFFFFFFFu, at, 1) + w.F;
+    if (pn + cn > NS + w.L.ncap || pf + cf > w.L.fcap) C.stop = WV_ERR_OVERFLOW;
+    if (lane == 0) w.npush += cn + cf;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint2 e = make_uint2(ed[u].x, nd[u]);
+      if ((bn[u] >> lane) & 1u) put(S, w, w.cur ^ 1u, pn + __popc(bn[u] & lt), e);
+      if ((bf[u] >> lane) & 1u) {
+        const unsigned i = pf + __popc(bf[u] & lt);
+        if (i < w.L.fcap) __stcg(w.L.far + i, e);
+      }
+      pn += __popc(bn[u]);
+      pf += __popc(bf[u]);
+    }
+  }
+
+  /* a lane's entry: its row (or its piece of a long row: ids from n up), and
+   * whether its distance is still the vertex's */
+  static __device__ __forceinline__ void load(const State &w, uint2 x, bool in, unsigned &r0,
+                                              unsigned &deg, bool &live) {
+    r0 = deg = 0u;
+    live = false;
+    if (in) {
+      unsigned v = x.x;
+      if (v < w.n) {
+        r0 = __ldg(w.row + v);
+        deg = __ldg(w.row + v + 1) - r0;
+      } else {
+        const uint4 c = __ldg(w.piece + (v - w.n));
+        v = c.x;
+        r0 = c.y;
+        deg = c.z;
+      }
+      live = __ldcg(w.dist + v) == x.y;
+    }
+  }
+
+  /* A long row becomes pieces of WV_PIECE edges in the next frontier, which
+   * an exchange deals out over the group (one warp on a row of thousands of
+   * edges would hold up the hop). */
+  static __device__ __forceinline__ void cut(Smem &S, State &w, uint2 x, unsigned deg) {
+    Ctr &C = S.ctr[next3(w.ci)];
+    const unsigned k = (deg + WV_PIECE - 1u) / WV_PIECE, c0 = w.n + __ldg(w.first + x.x);
+    const unsigned at = atomicAdd(&C.near_cnt, k);
+    if (at + k > NS + w.L.ncap) C.stop = WV_ERR_OVERFLOW;
+    C.cut = 1u;
+    for (unsigned j = 0; j < k; ++j) put(S, w, w.cur ^ 1u, at + j, make_uint2(c0 + j, x.y));
+  }
+
+  /* The edges of up to 32 entries (one a lane) spread over the warp: 32
+   * neighbouring edges per load, a lane's row found by a search over the
+   * row offsets. */
+  static __device__ __forceinline__ void spread(Smem &S, State &w, uint2 x, unsigned r0,
+                                                unsigned deg) {
+    constexpr int U = 4;
+    const unsigned lane = threadIdx.x & 31u;
+    unsigned off = deg;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xFFFFFFFFu, off, o);
+      if (lane >= (unsigned)o) off += y;
+    }
+    const unsigned E = __shfl_sync(0xFFFFFFFFu, off, 31);
+    off -= deg;
+    if (lane == 0) w.nedge += E;
+    for (unsigned e0 = 0; e0 < E; e0 += 32u * U) {
+      uint2 e[U];
+      unsigned dd[U], msk = 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned k = e0 + u * 32u + lane;
+        unsigned j = 0;
+#pragma unroll
+        for (int b = 16; b > 0; b >>= 1) {
+          const unsigned o = __shfl_sync(0xFFFFFFFFu, off, j + b);
+          if (o <= k) j += b;
+        }
+        const unsigned ro = __shfl_sync(0xFFFFFFFFu, r0, j);
+        const unsigned oo = __shfl_sync(0xFFFFFFFFu, off, j);
+        dd[u] = __shfl_sync(0xFFFFFFFFu, x.y, j);
+        e[u] = make_uint2(0u, 0u);
+        if (k < E) {
+          e[u] = __ldg(w.edges + ro + (k - oo));
+          msk |= 1u << u;
+        }
+      }
+      relax<U>(S, w, e, dd, msk);
+    }
+  }
+
+  /* A hop whose edges are pooled over the CTA: a block scan of the row
+   * lengths, then every warp walks 32 x U neighbouring edges at a time. */
+  static __device__ __forceinline__ void hop_pool(Smem &S, State &w, unsigned cnt) {
+    constexpr int U = 4;
+    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    if (tid == 0) S.ctr[next3(next3(w.ci))] = Ctr{0u, 0u, 0u, 0u};
+    for (unsigned i0 = 0; i0 < cnt; i0 += BLOCK) {
+      const bool in = i0 + tid < cnt;
+      const uint2 x = in ? entry(S, w, i0 + tid) : make_uint2(0u, 0u);
+      unsigned r0, deg;
+      bool live;
+      load(w, x, in, r0, deg, live);
+      if (in && !live) ++w.nstale;
+      if (deg > WV_PIECE && x.x < w.n) {
+        if (live) cut(S, w, x, deg);
+        deg = 0u;
+      }
+      if (!live) deg = 0u;
+      unsigned off = deg;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xFFFFFFFFu, off, o);
+        if (lane >= (unsigned)o) off += y;
+      }
+      if (lane == 31u) S.wsum[warp] = off;
+      S.it_r0[tid] = r0;
+      S.it_d[tid] = x.y;
+      __syncthreads();
+      unsigned ws = lane < BLOCK / 32u ? S.wsum[lane] : 0u;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xFFFFFFFFu, ws, o);
+        if (lane >= (unsigned)o) ws += y;
+      }
+      const unsigned E = __shfl_sync(0xFFFFFFFFu, ws, 31);
+      const unsigned wb = __shfl_sync(0xFFFFFFFFu, ws, (warp + 31u) & 31u);
+      S.it_off[tid] = off - deg + (warp ? wb : 0u);
+      if (tid == 0) S.it_off[BLOCK] = E;
+      w.nedge += deg;
+      __syncthreads();
+      const unsigned k = min((unsigned)BLOCK, cnt - i0);
+      /* each warp a run of neighbouring edges: a lane's next edge is 32 further,
+       * so its row is at most a few items on */
+      const unsigned run = ((E + BLOCK / 32u - 1u) / (BLOCK / 32u) + 31u) & ~31u;
+      const unsigned re = min(E, (warp + 1u) * run);
+      unsigned lo = 0; /* item of the lane's last edge: its edges only move forward */
+      for (unsigned e0 = warp * run; e0 < re; e0 += 32u * U) {
+        uint2 e[U];
+        unsigned dd[U], msk = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const unsigned j = e0 + u * 32u + lane;
+          e[u] = make_uint2(0u, 0u);
+          dd[u] = 0u;
+          if (j < re) {
+            unsigned step = 1u;
+            while (lo + step < k && S.it_off[lo + step] <= j) {
+              lo += step;
+              step <<= 1;
+            }
+            unsigned hi = min(lo + step, k) - 1u;
+            while (lo < hi) {
+              const unsigned mid = (lo + hi + 1u) >> 1;
+              if (S.it_off[mid] <= j) lo = mid; else hi = mid - 1u;
+            }
+            e[u] = __ldg(w.edges + S.it_r0[lo] + (j - S.it_off[lo]));
+            dd[u] = S.it_d[lo];
+            msk |= 1u << u;
+          }
+        }
+        relax<U>(S, w, e, dd, msk);
+      }
+      __syncthreads(); /* the pool is read */
+    }
+  }
+
+  /* One hop: relaxes the rows of the cnt frontier entries into the next
+   * frontier and the far list.  The caller's barrier ends it. */
+  static __device__ __forceinline__ void hop(Smem &S, State &w, unsigned cnt) {
+    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    if (tid == 0) S.ctr[next3(next3(w.ci))] = Ctr{0u, 0u, 0u, 0u};
+    /* few entries: eight a warp, four lanes each, rows of up to eight edges in
+     * one round, so that every warp of the CTA has part of the hop */
+    const bool few = cnt <= BLOCK / 4u;
+    for (unsigned i0 = warp * (few ? 8u : 32u); i0 < cnt; i0 += BLOCK) {
+      const unsigned i = i0 + (few ? lane >> 2 : lane);
+      const bool in = i < cnt, first = !few || (lane & 3u) == 0u;
+      const uint2 x = in ? entry(S, w, i) : make_uint2(0u, 0u);
+      unsigned r0, deg;
+      bool live;
+      load(w, x, in, r0, deg, live);
+      if (first && in && !live) ++w.nstale;
+      if (deg > WV_PIECE && x.x < w.n) {
+        if (live && first) cut(S, w, x, deg);
+        deg = 0u;
+      }
+      if (GRP && few && __reduce_max_sync(0xFFFFFFFFu, deg) <= 8u) {
+        uint2 e[2];
+        const unsigned dd[2] = {x.y, x.y};
+        unsigned msk = 0;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const unsigned k = u * 4u + (lane & 3u);
+          e[u] = make_uint2(0u, 0u);
+          if (k < deg) { /* read before it is known whether the entry is live */
+            e[u] = __ldg(w.edges + r0 + k);
+            msk |= 1u << u;
+          }
+        }
+        if (!live) msk = 0;
+        if (live && first) w.nedge += deg;
+        relax<2>(S, w, e, dd, msk, true);
+        continue;
+      }
+      if (!live) deg = 0u;
+      const unsigned maxdeg = __reduce_max_sync(0xFFFFFFFFu, deg);
+      if (maxdeg <= 8u) {
+        /* short rows: four lanes to a vertex, eight vertices to a load, so
+         * that a row's edges come with one request */
+        if (first) w.nedge += deg;
+        for (unsigned k0 = 0; k0 < maxdeg; k0 += 4u) {
+          const unsigned k = k0 + (lane & 3u);
+          if (few) {
+            const uint2 e[1] = {k < deg ? __ldg(w.edges + r0 + k) : make_uint2(0u, 0u)};
+            const unsigned dd[1] = {x.y};
+            relax<1>(S, w, e, dd, k < deg ? 1u : 0u);
+            continue;
+          }
+          uint2 e[4];
+          unsigned dd[4], msk = 0;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int own = u * 8 + (int)(lane >> 2);
+            const unsigned ro = __shfl_sync(0xFFFFFFFFu, r0, own);
+            const unsigned dg = __shfl_sync(0xFFFFFFFFu, deg, own);
+            dd[u] = __shfl_sync(0xFFFFFFFFu, x.y, own);
+            e[u] = make_uint2(0u, 0u);
+            if (k < dg) {
+              e[u] = __ldg(w.edges + ro + k);
+              msk |= 1u << u;
+            }
+          }
+          relax<4>(S, w, e, dd, msk);
+        }
+      } else {
+        spread(S, w, x, r0, first ? deg : 0u);
+      }
+    }
+  }
+
+  /* Moves T up and splits this CTA's far list against it: entries below join
+   * the frontier, stale ones are dropped, the others are packed in place (a
+   * tile is read before any of it is written over).  Uniform over the CTA;
+   * the counter's frontier count and w.F are current afterwards. */
+  static __device__ void split(Smem &S, State &w) {
+    const unsigned tid = threadIdx.x, lane = tid & 31u, lt = (1u << lane) - 1u;
+    Ctr &C = S.ctr[w.ci];
+    if (tid == 0) {
+      S.kept = 0u;
+      S.fmin = 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    unsigned lmin = 0xFFFFFFFFu;
+    for (unsigned i0 = 0; i0 < w.F; i0 += BLOCK * 2u) {
+      uint2 x[2];
+      bool in[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const unsigned i = i0 + u * BLOCK + tid;
+        in[u] = i < w.F;
+        x[u] = in[u] ? __ldcg(w.L.far + i) : make_uint2(0u, 0u);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (in[u] && __ldcg(w.dist + x[u].x) != x[u].y) {
+          in[u] = false;
+          ++w.nstale;
+        }
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const bool nr = x[u].y < w.T;
+        const unsigned bn = __ballot_sync(0xFFFFFFFFu, in[u] && nr);
+        const unsigned bf = __ballot_sync(0xFFFFFFFFu, in[u] && !nr);
+        if ((bn | bf) == 0u) continue;
+        unsigned at = 0;
+        if (lane < 2u) at = atomicAdd(lane ? &S.kept : &C.near_cnt, (unsigned)__popc(lane ? bf : bn));
+        const unsigned pn = __shfl_sync(0xFFFFFFFFu, at, 0), pf = __shfl_sync(0xFFFFFFFFu, at, 1);
+        if (pn + __popc(bn) > NS + w.L.ncap) C.stop = WV_ERR_OVERFLOW;
+        if ((bn >> lane) & 1u) put(S, w, w.cur, pn + __popc(bn & lt), x[u]);
+        if ((bf >> lane) & 1u) {
+          __stcg(w.L.far + pf + __popc(bf & lt), x[u]);
+          lmin = min(lmin, x[u].y);
+        }
+      }
+    }
+    lmin = __reduce_min_sync(0xFFFFFFFFu, lmin);
+    if (lane == 0 && lmin != 0xFFFFFFFFu) atomicMin(&S.fmin, lmin);
+    __syncthreads();
+    w.F = S.kept;
+  }
+
+  /* Group exchange: every CTA publishes its frontier and its counts, and
+   * takes an equal, contiguous share of the whole frontier back as its own
+   * (neighbouring vertices stay together, so the hops that follow seldom
+   * improve a vertex of another CTA).  False when the launch must end. */
+  static __device__ bool exchange(const WvParams &P, Smem &S, State &w, unsigned cnt,
+                                  unsigned fmin, unsigned stop, unsigned &round,
+                                  unsigned long long deadline) {
+    const unsigned tid = threadIdx.x, lane = tid & 31u, rank = blockIdx.x, G = P.gsize;
+    const unsigned par = round & 1u, xcap = NS + w.L.ncap;
+    /* areas are the same size for every CTA of a group */
+    const size_t stride = 2ull * w.L.ncap + w.L.fcap + 2ull * xcap;
+    uint2 *const mine = w.L.far + w.L.fcap + (size_t)par * xcap;
+    for (unsigned i = tid; i < min(cnt, xcap); i += BLOCK) __stcg(mine + i, entry(S, w, i));
+    __syncthreads();
+    /* The CTA's note carries the round: it is the arrival too.  One warp reads
+     * every CTA's note until all are of this round.  Notes and published
+     * frontiers alternate between two areas, so a CTA that runs ahead does not
+     * write over what a slower one still reads. */
+    ulonglong2 *const notes =
+        reinterpret_cast<ulonglong2 *>(P.grp) + (size_t)par * WV_MAX_GROUP;
+    ++round;
+    const unsigned tag = round << 2; /* low bits: the error */
+    if (tid < 32u) {
+      if (lane == 0) {
+        __threadfence(); /* what the CTA published, before its note */
+        st_note(notes + rank, min(cnt, xcap), w.F, fmin, tag | stop);
+      }
+      constexpr unsigned J = WV_MAX_GROUP / 32u;
+      unsigned c[J], far = 0, fm = 0xFFFFFFFFu, st = 0, it = 0;
+      bool late = false;
+      for (;;) {
+        far = st = 0u;
+        fm = 0xFFFFFFFFu;
+        bool here = true;
+#pragma unroll
+        for (unsigned j = 0; j < J; ++j) {
+          const unsigned r = j * 32u + lane;
+          uint4 x = make_uint4(0u, 0u, 0xFFFFFFFFu, tag);
+          if (r < G) x = ld_note(notes + r);
+          here = here && (x.w & ~3u) == tag;
+          c[j] = x.x;
+          far += x.y;
+          fm = min(fm, x.z);
+          st = max(st, x.w & 3u);
+        }
+        if (__all_sync(0xFFFFFFFFu, here)) break;
+        late = (++it & 255u) == 0u && gtimer() > deadline;
+        if (__any_sync(0xFFFFFFFFu, late)) break;
+      }
+      late = __any_sync(0xFFFFFFFFu, late);
+      __threadfence(); /* the notes, before what they announce */
+      unsigned tot = 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+        for (unsigned j = 0; j < J; ++j) {
+          const unsigned y = __shfl_up_sync(0xFFFFFFFFu, c[j], o);
+          if (lane >= (unsigned)o) c[j] += y;
+        }
+      }
+#pragma unroll
+      for (unsigned j = 0; j < J; ++j) {
+        c[j] += tot;
+        tot = __shfl_sync(0xFFFFFFFFu, c[j], 31);
+        if (j * 32u + lane < G) S.pre[j * 32u + lane] = c[j];
+      }
+      far = __reduce_add_sync(0xFFFFFFFFu, far);
+      fm = __reduce_min_sync(0xFFFFFFFFu, fm);
+      st = __reduce_max_sync(0xFFFFFFFFu, st);
+      /* first CTA whose entries reach into this CTA's share */
+      const unsigned shr = ((tot + G - 1u) / G + 7u) & ~7u, lo = min(rank * shr, tot);
+      unsigned first = 0;
+#pragma unroll
+      for (unsigned j = 0; j < J; ++j)
+        first += __popc(__ballot_sync(0xFFFFFFFFu, j * 32u + lane < G && c[j] <= lo));
+      if (lane == 0) {
+        S.tot = Note{tot, far, fm, st};
+        S.r0 = min(first, G - 1u);
+        S.q = late ? 1u : 0u;
+        if (late) atomicCAS(&P.st->err, 0u, WV_ERR_TIMEOUT);
+      }
+    }
+    __syncthreads();
+    if (S.q != 0u) return false; /* the wait ran out */
+    const unsigned tot = S.tot.near_cnt;
+    const unsigned shr = ((tot + G - 1u) / G + 7u) & ~7u;
+    unsigned lo = min(rank * shr, tot), hi = min(lo + shr, tot), step = 1u, r = S.r0;
+    if (POOL) { /* dealt out one by one: a long row's pieces lie together */
+      lo = rank;
+      hi = rank + (tot > rank ? (tot - rank + G - 1u) / G : 0u);
+      step = G;
+      r = 0u;
+    }
+    const uint2 *const base = reinterpret_cast<const uint2 *>(P.ws) + 2ull * w.L.ncap + w.L.fcap +
+                              (size_t)par * xcap;
+    for (unsigned j = tid; j < hi - lo; j += BLOCK) {
+      const unsigned i = lo + j * step; /* below tot = pre[G - 1] */
+      if (POOL) {
+        unsigned top = G - 1u;
+        while (r < top) {
+          const unsigned mid = (r + top) >> 1;
+          if (S.pre[mid] <= i) r = mid + 1u; else top = mid;
+        }
+      } else {
+        while (S.pre[r] <= i) ++r;
+      }
+      put(S, w, w.cur, j, __ldcg(base + r * stride + (i - (r ? S.pre[r - 1] : 0u))));
+    }
+    if (tid == 0) {
+      S.ctr[w.ci] = Ctr{hi - lo, 0u, 0u, 0u};
+      S.ctr[next3(w.ci)] = Ctr{0u, 0u, 0u, 0u};
+      if (hi - lo > NS + w.L.ncap) S.ctr[w.ci].stop = WV_ERR_OVERFLOW;
+    }
+    __syncthreads();
+    return true;
+  }
+
+  static __device__ void run(const WvParams &P, Smem &S) {
+    const unsigned tid = threadIdx.x, lane = tid & 31u;
+    const WvArea A = P.area[blockIdx.x];
+    const unsigned inf = FLT ? ADDS_INF_F32_BITSV : ADDS_INF_I32_BITS;
+    const unsigned long long deadline = gtimer() + P.timeout_ns;
+    unsigned long long s_items = 0, s_hops = 0, s_splits = 0;
+    State w;
+    w.L.over = reinterpret_cast<uint2 *>(P.ws) + A.off;
+    w.L.far = w.L.over + 2ull * A.ncap;
+    w.L.ncap = A.ncap;
+    w.L.fcap = A.fcap;
+    w.npush = w.nstale = 0u;
+    w.nedge = 0ull;
+    unsigned err0 = *reinterpret_cast<volatile unsigned *>(&P.st->err), round = 0;
+    for (unsigned turn = 0;; ++turn) {
+      /* a CTA's next query: its own first, then from the counter */
+      if (tid == 0) {
+        const unsigned i = GRP ? turn : (turn == 0 ? blockIdx.x : atomicAdd(&P.st->next, 1u) + P.groups);
+        S.q = i < P.nq ? P.order[i] : 0xFFFFFFFFu;
+        S.ctr[0] = Ctr{GRP && blockIdx.x != 0u ? 0u : 1u, 0u, err0, 0u};
+        S.ctr[1] = S.ctr[2] = Ctr{0u, 0u, 0u, 0u};
+      }
+      __syncthreads();
+      const unsigned q = S.q;
+      if (q == 0xFFFFFFFFu) break;
+      const WvQuery Q = P.qs[q];
+      w.row = Q.row;
+      w.edges = Q.edges;
+      w.first = Q.first;
+      w.piece = Q.piece;
+      w.dist = Q.dist;
+      w.n = Q.n;
+      const unsigned src = (P.single_src != 0xFFFFFFFFu && q == 0u) ? P.single_src : Q.src;
+      if (!GRP && !P.filled) {
+        if ((reinterpret_cast<unsigned long long>(Q.dist) & 15ull) == 0ull) {
+          const unsigned n4 = Q.n >> 2;
+          for (unsigned i = tid; i < n4; i += BLOCK)
+            __stcg(reinterpret_cast<uint4 *>(Q.dist) + i, make_uint4(inf, inf, inf, inf));
+          if (tid < (Q.n & 3u)) __stcg(Q.dist + (n4 << 2) + tid, inf);
+        } else {
+          for (unsigned i = tid; i < Q.n; i += BLOCK) __stcg(Q.dist + i, inf);
+        }
+        __syncthreads();
+        if (tid == 0) __stcg(Q.dist + src, 0u);
+      }
+      if (tid == 0) S.nb[0][0] = make_uint2(src, 0u);
+      __syncthreads();
+      float delta = Q.delta;
+      w.T = raise_word<FLT>(0u, delta);
+      w.cur = w.ci = w.F = 0u;
+      unsigned fmin = 0xFFFFFFFFu, hops = 0, split_at = 0, stop = 0;
+      if (!GRP) {
+        for (;;) {
+          const Ctr c = S.ctr[w.ci];
+          w.F += c.far_new;
+          unsigned cnt = c.near_cnt;
+          stop = c.stop;
+          if (stop != 0u) break;
+          if (cnt <= P.low && w.F != 0u) {
+            /* a frontier that ran low again within a few hops: a wider step */
+            if (hops - split_at <= 4u) delta *= 1.5f;
+            split_at = hops;
+            w.T = raise_word<FLT>(cnt == 0u && fmin != 0xFFFFFFFFu && fmin > w.T ? fmin : w.T, delta);
+            split(S, w);
+            fmin = S.fmin;
+            cnt = S.ctr[w.ci].near_cnt;
+            stop = S.ctr[w.ci].stop;
+            __syncthreads();
+            if (tid == 0) S.ctr[w.ci].far_new = 0u; /* in w.F already */
+            ++s_splits;
+            if (stop != 0u) break;
+            if (cnt == 0u) {
+              __syncthreads();
+              if (w.F == 0u) break;
+              continue;
+            }
+          }
+          if (cnt == 0u) break;
+          if (cnt > P.high) delta *= 0.75f;
+          s_items += cnt;
+          if (POOL) hop_pool(S, w, cnt); else hop(S, w, cnt);
+          ++hops;
+          if (tid == 0 && (hops & 1023u) == 0u && gtimer() > deadline)
+            S.ctr[next3(w.ci)].stop = WV_ERR_TIMEOUT;
+          __syncthreads();
+          w.cur ^= 1u;
+          w.ci = next3(w.ci);
+        }
+      } else {
+        for (;;) {
+          /* up to P.hops hops on this CTA's own entries */
+          unsigned cnt = 0;
+          for (unsigned h = 0;; ++h) {
+            const Ctr c = S.ctr[w.ci];
+            w.F += c.far_new;
+            cnt = c.near_cnt;
+            stop = c.stop;
+            if (h == P.hops || cnt == 0u || stop != 0u || (h != 0u && (cnt > BLOCK / 2u || c.cut != 0u)))
+              break;
+            s_items += cnt;
+            if (POOL) hop_pool(S, w, cnt); else hop(S, w, cnt);
+            ++hops;
+            __syncthreads();
+            w.cur ^= 1u;
+            w.ci = next3(w.ci);
+          }
+          if (!exchange(P, S, w, cnt, fmin, stop, round, deadline)) {
+            stop = WV_ERR_TIMEOUT;
+            break;
+          }
+          const Note t = S.tot;
+          stop = t.stop;
+          if (stop != 0u || (t.near_cnt == 0u && t.far_cnt == 0u)) break;
+          if (t.near_cnt <= P.low && t.far_cnt != 0u) {
+            if (round - split_at <= 1u) delta *= 1.5f;
+            split_at = round;
+            w.T = raise_word<FLT>(
+                t.near_cnt == 0u && t.far_min != 0xFFFFFFFFu && t.far_min > w.T ? t.far_min : w.T, delta);
+            split(S, w);
+            fmin = S.fmin;
+            ++s_splits;
+          } else if (t.near_cnt > P.high) {
+            delta *= 0.75f;
+          }
+          __syncthreads();
+          if (gtimer() > deadline && tid == 0 && blockIdx.x == 0) S.ctr[w.ci].stop = WV_ERR_TIMEOUT;
+          __syncthreads();
+        }
+      }
+      s_hops += hops;
+      if (stop != 0u && tid == 0) atomicCAS(&P.st->err, 0u, stop);
+      __syncthreads(); /* S is read to the end before the next query's setup */
+      if (stop != 0u) break;
+    }
+    unsigned long long s_edge = w.nedge, s_push = w.npush, s_stale = w.nstale;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s_edge += __shfl_down_sync(0xFFFFFFFFu, s_edge, o);
+      s_push += __shfl_down_sync(0xFFFFFFFFu, s_push, o);
+      s_stale += __shfl_down_sync(0xFFFFFFFFu, s_stale, o);
+    }
+    if (lane == 0) {
+      if (s_edge) atomicAdd(&P.st->edges, s_edge);
+      if (s_push) atomicAdd(&P.st->pushes, s_push);
+      if (s_stale) atomicAdd(&P.st->stale, s_stale);
+      if (tid == 0) {
+        atomicAdd(&P.st->items, s_items);
+        if (!GRP || blockIdx.x == 0u) {
+          atomicAdd(&P.st->steps, GRP ? (unsigned long long)round : s_hops);
+          atomicAdd(&P.st->splits, s_splits);
+        }
+      }
+    }
+  }
+};
+
+template <bool FLT, int BLOCK, int NS, int MINB, bool GRP, bool POOL>
+__global__ void __launch_bounds__(BLOCK, MINB) wave_kernel(const __grid_constant__ WvParams P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Wave<FLT, BLOCK, NS, GRP, POOL>::run(P, *reinterpret_cast<WSmem<BLOCK, NS, POOL> *>(smem_raw));
+}
+
+/* INF everywhere and 0 at the source, by the whole GPU */
+__global__ void wave_fill(const WvQuery *qs, unsigned single_src, unsigned inf) {
+  const WvQuery Q = qs[0];
+  const unsigned src = single_src != 0xFFFFFFFFu ? single_src : Q.src;
+  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < Q.n; v += gridDim.x * blockDim.x)
+    Q.dist[v] = v == src ? 0u : inf;
+}
+
+template <bool FLT, int BLOCK, int NS, int MINB, bool GRP, bool POOL>
+static cudaError_t resident(int *bps) {
+  const int smem = (int)sizeof(WSmem<BLOCK, NS, POOL>);
+  auto *k = wave_kernel<FLT, BLOCK, NS, MINB, GRP, POOL>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k, BLOCK, smem);
+}
+
+template <bool FLT, int BLOCK, int NS, int MINB, bool GRP, bool POOL>
+static cudaError_t launch(const WvParams &P, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(P.groups * P.gsize);
+  cfg.blockDim = dim3(BLOCK);
+  cfg.dynamicSmemBytes = sizeof(WSmem<BLOCK, NS, POOL>);
+  cfg.stream = st;
+  /* the CTAs of a group wait for each other: all must be resident */
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = GRP ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, wave_kernel<FLT, BLOCK, NS, MINB, GRP, POOL>, P);
+}
+
+}  // namespace adds_wave
+
+/* (variant, threads, frontier entries in shared memory, CTAs per SM the
+ * registers are sized for, several CTAs per query, pooled edges, entries per
+ * CTA below which a frontier takes more of the far list).  The batch of 128
+ * grids x 16 sources: 256 threads x 4 7.2 ms, x 5 7.6, x 6 8.2, 128 x 10 11.4,
+ * 512 x 3 7.8, 1024 x 1 14.5.  Low marks: 32 entries 7.6 ms, 16 7.7, 64 8.0, 0
+ * 8.2 there; 4096^2 grid on 148 CTAs 2,500 entries 18.3 ms, 1,000 19.3, 9,500
+ * 21.7. */
+#define WV_SHAPES(X)                           \
+  X(WV_CTA, 256, 1024, 4, false, false, 32)    \
+  X(WV_WIDE, 1024, 4096, 1, false, false, 64)  \
+  X(WV_GROUP, 512, 2048, 1, true, false, 16)   \
+  X(WV_POOL, 512, 2048, 1, true, true, 8)
+
+static unsigned wv_block(int shape) {
+#define X(s, b, ns, m, g, pl, lo) if (shape == s) return b;
+  WV_SHAPES(X)
+#undef X
+  return 0;
+}
+static unsigned wv_low(int shape) {
+#define X(s, b, ns, m, g, pl, lo) if (shape == s) return lo;
+  WV_SHAPES(X)
+#undef X
+  return 0;
+}
+static unsigned wv_near(int shape) {
+#define X(s, b, ns, m, g, pl, lo) if (shape == s) return ns;
+  WV_SHAPES(X)
+#undef X
+  return 0;
+}
+
+void wv_engine_free(WvEngine &E) {
+  void *ptrs[] = {E.qs, E.order, E.area, E.ws, E.st, E.grp};
+  for (void *p : ptrs)
+    if (p) cudaFree(p);
+  if (E.st_host) cudaFreeHost(E.st_host);
+  E = WvEngine();
+}
+
+int wv_engine_reset(WvEngine &E, cudaStream_t st) {
+  return cudaMemsetAsync(E.st, 0, sizeof(WvStat), st) == cudaSuccess &&
+                 cudaStreamSynchronize(st) == cudaSuccess
+             ? 0
+             : -5;
+}
+
+int wv_engine_upload(WvEngine &E, cudaStream_t st) {
+  return cudaMemcpyAsync(E.qs, E.qs_host.data(), E.qs_host.size() * sizeof(WvQuery),
+                         cudaMemcpyHostToDevice, st) == cudaSuccess &&
+                 cudaStreamSynchronize(st) == cudaSuccess
+             ? 0
+             : -5;
+}
+
+/* gsize: CTAs per query of the WV_GROUP variant (0: one per SM) */
+int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize,
+                    const std::vector<WvQuery> &qv, cudaStream_t st) {
+  using namespace adds_wave;
+  wv_engine_free(E);
+  E.device = device;
+  E.flt = flt;
+  E.shape = shape;
+  E.nq = (unsigned)qv.size();
+  E.qs_host = qv;
+  int sms = 0, bps = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+    return -5;
+  cudaError_t e = cudaErrorInvalidValue;
+#define X(s, b, ns, m, g, pl, lo) \
+  if (shape == s)         \
+    e = flt ? resident<true, b, ns, m, g, pl>(&bps) : resident<false, b, ns, m, g, pl>(&bps);
+  WV_SHAPES(X)
+#undef X
+  if (e != cudaSuccess || bps < 1) {
+    cudaGetLastError();
+    return -9;
+  }
+  const bool grp = shape == WV_GROUP || shape == WV_POOL;
+  if (grp && E.nq != 1u) return -9;
+  E.gsize = grp ? std::min(gsize ? gsize : (unsigned)sms, std::min((unsigned)sms, (unsigned)WV_MAX_GROUP)) : 1u;
+  E.req_gsize = gsize;
+  E.groups = grp ? 1u : std::min((unsigned)(bps * sms), E.nq);
+  E.ctas = E.groups * E.gsize;
+  /* largest first: the last group to finish is not stuck with a big query */
+  std::vector<unsigned> order(E.nq);
+  for (unsigned i = 0; i < E.nq; ++i) order[i] = i;
+  std::stable_sort(order.begin(), order.end(), [&](unsigned a, unsigned b) {
+    return qv[a].m + qv[a].n > qv[b].m + qv[b].n;
+  });
+  /* A CTA's lists hold the queries it may meet: its own first one and any
+   * later one.  A road's wave front is a small part of its graph: frontier
+   * n/4 (and the shared entries) and far list n/2 in all.  A graph with longer
+   * rows has most of its vertices pending at once, some of them several times.
+   * Either way one CTA may hold much more than its share for a few hops.
+   * Where that is not enough, the launch reports an overflow. */
+  bool dense = false;
+  for (const WvQuery &q : qv) dense = dense || q.m >= 6ull * q.n;
+  std::vector<WvArea> area;
+  std::vector<unsigned> maxn(E.nq);
+  for (unsigned i = E.nq, mx = 0; i-- > 0;) {
+    mx = std::max(mx, qv[order[i]].n);
+    maxn[i] = mx;
+  }
+  unsigned long long tot = 0;
+  for (;;) {
+    area.clear();
+    tot = 0;
+    for (unsigned g = 0; g < E.groups; ++g)
+      for (unsigned r = 0; r < E.gsize; ++r) {
+        const unsigned long long n = maxn[g], cl = E.gsize;
+        WvArea A;
+        A.off = tot;
+        A.ncap = (unsigned)((dense ? n : n / 4u) / cl + std::min(n, 16384ull));
+        A.fcap = (unsigned)((dense ? 4u * n : n / 2u) / cl + std::min(2ull * n, 65536ull));
+        tot += 2ull * A.ncap + A.fcap;
+        if (grp) tot += 2ull * (wv_near(shape) + A.ncap); /* published frontiers */
+        area.push_back(A);
+      }
+    /* at most 8 GB of lists: fewer queries side by side, if need be */
+    if (tot <= (1ull << 30)) break;
+    if (E.groups <= 8u) return -4;
+    E.groups /= 2u;
+  }
+  E.ctas = E.groups * E.gsize;
+#define WV_ALLOC(ptr, bytes_)                             \
+  do {                                                    \
+    const size_t _b = (bytes_);                           \
+    if (cudaMalloc((void **)&(ptr), _b) != cudaSuccess) { \
+      cudaGetLastError();                                 \
+      wv_engine_free(E);                                  \
+      return -4;                                          \
+    }                                                     \
+    E.bytes += _b;                                        \
+  } while (0)
+  WV_ALLOC(E.qs, (size_t)E.nq * sizeof(WvQuery));
+  WV_ALLOC(E.order, (size_t)E.nq * 4);
+  WV_ALLOC(E.area, (size_t)E.ctas * sizeof(WvArea));
+  WV_ALLOC(E.ws, (size_t)tot * 8);
+  WV_ALLOC(E.st, sizeof(WvStat));
+  WV_ALLOC(E.grp, WV_GRP_WORDS * 4);
+#undef WV_ALLOC
+  if (cudaMallocHost((void **)&E.st_host, sizeof(WvStat)) != cudaSuccess) {
+    cudaGetLastError();
+    wv_engine_free(E);
+    return -4;
+  }
+  memset(E.st_host, 0, sizeof(WvStat));
+  if (cudaMemcpyAsync(E.order, order.data(), (size_t)E.nq * 4, cudaMemcpyHostToDevice, st) !=
+          cudaSuccess ||
+      cudaMemcpyAsync(E.area, area.data(), area.size() * sizeof(WvArea), cudaMemcpyHostToDevice,
+                      st) != cudaSuccess)
+    return -5;
+  const int rc = wv_engine_upload(E, st);
+  return rc ? rc : wv_engine_reset(E, st);
+}
+
+int wv_engine_enqueue(WvEngine &E, unsigned single_src, unsigned long long timeout_ns,
+                      cudaStream_t st, cudaEvent_t k0, cudaEvent_t k1) {
+  using namespace adds_wave;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) return -5;
+  const unsigned fl = cs == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0u;
+  const size_t keep = offsetof(WvStat, next); /* the error word stays */
+  if (cudaMemsetAsync(reinterpret_cast<char *>(E.st) + keep, 0, sizeof(WvStat) - keep, st) !=
+      cudaSuccess)
+    return -5;
+  WvParams P;
+  memset(&P, 0, sizeof P);
+  P.qs = E.qs;
+  P.order = E.order;
+  P.nq = E.nq;
+  P.groups = E.groups;
+  P.gsize = E.gsize;
+  P.area = E.area;
+  P.ws = E.ws;
+  P.st = E.st;
+  P.grp = E.grp;
+  P.single_src = single_src;
+  P.timeout_ns = timeout_ns;
+  P.low = wv_low(E.shape) * E.gsize;
+  P.high = wv_block(E.shape) * E.gsize * 4u;
+  /* Hops on a CTA's own entries between two exchanges.  Roads: 8 (a 4096^2
+   * grid 18.3 ms, against 19.3 at 4 and 33 at 1, where the exchanges cost more
+   * than the hops).  Pooled: 1, since the neighbours of an entry are anywhere
+   * and hops on stale distances relax too much (R-MAT 16 0.38 ms, 0.60 at 8),
+   * but 8 on graphs so small that the few hops are all there is (20,000
+   * vertices 0.20 ms, 0.27 at 1). */
+  P.hops = E.shape == WV_GROUP || (E.qs_host[0].n < 32768u && !E.qs_host[0].piece) ? 8u : 1u;
+  const bool grp = E.shape == WV_GROUP || E.shape == WV_POOL;
+  P.filled = grp || (E.nq == 1u && E.qs_host[0].n > (1u << 18)) ? 1u : 0u;
+  if (grp && cudaMemsetAsync(E.grp, 0, WV_GRP_WORDS * 4, st) != cudaSuccess) return -5;
+  if (P.filled)
+    wave_fill<<<1184, 256, 0, st>>>(E.qs, single_src,
+                                    E.flt ? ADDS_INF_F32_BITSV : ADDS_INF_I32_BITS);
+  if (k0 && cudaEventRecordWithFlags(k0, st, fl) != cudaSuccess) return -5;
+  cudaError_t e = cudaErrorInvalidValue;
+#define X(s, b, ns, m, g, pl, lo) \
+  if (E.shape == s) e = E.flt ? launch<true, b, ns, m, g, pl>(P, st) : launch<false, b, ns, m, g, pl>(P, st);
+  WV_SHAPES(X)
+#undef X
+  if (e != cudaSuccess) return -5;
+  if (k1 && cudaEventRecordWithFlags(k1, st, fl) != cudaSuccess) return -5;
+  if (cudaMemcpyAsync(E.st_host, E.st, sizeof(WvStat), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+    return -5;
+  return 0;
+}
+
+int wv_engine_status(const WvEngine &E, char *msg, size_t msg_len) {
+  const unsigned err = E.st_host->err;
+  if (err && msg) snprintf(msg, msg_len, "wave kernel: device error %u", err);
+  return err == 0u ? 0 : (err == WV_ERR_OVERFLOW ? -7 : -6);
+}

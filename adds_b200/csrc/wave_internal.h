@@ -1,0 +1,105 @@
+/*
+ * wave_internal.h — device data layout of the wave kernels (wave.cu).
+ *
+ * One group (a CTA, or a thread-block cluster) solves one query with two
+ * kinds of lists: the frontier of the current step, kept in shared memory
+ * with an overflow area in HBM, and a far list per CTA in HBM.  No page
+ * pool, no bucket ring, no barrier through memory.
+ */
+#ifndef ADDS_WAVE_INTERNAL_H_
+#define ADDS_WAVE_INTERNAL_H_
+
+#include <stdint.h>
+
+/* error word of a launch (first one wins) */
+#define WV_ERR_OVERFLOW 1u /* a list outgrew its area: solve on another engine */
+#define WV_ERR_TIMEOUT 2u
+
+#define WV_PIECE 512u     /* edges of a long row one entry stands for          */
+#define WV_MAX_GROUP 160u /* CTAs of one group (a multiple of 32)              */
+#define WV_GRP_WORDS (2u * 4u * WV_MAX_GROUP) /* two sets of 16-byte notes     */
+
+struct WvQuery {
+  const unsigned *row;
+  const uint2 *edges; /* rows in CSR order: nothing is sorted by weight        */
+  /* rows of more than WV_PIECE edges: their first piece by vertex, and the
+   * pieces {vertex, first edge, edges, 0}; null where no row is that long */
+  const unsigned *first;
+  const uint4 *piece;
+  unsigned *dist;
+  unsigned n;
+  unsigned src;
+  float delta;        /* first step of the near threshold, in distance units   */
+  unsigned pad;
+  unsigned long long m;
+};
+
+/* list areas of one CTA, in 16-byte entries from WvParams::ws */
+struct WvArea {
+  unsigned long long off; /* two frontier overflow areas, then the far list    */
+  unsigned ncap, fcap;    /* entries of one frontier overflow area / far list  */
+};
+
+struct WvStat {
+  unsigned err;           /* kept until the host resets the engine             */
+  unsigned pad0[31];
+  unsigned next;          /* batch: next query (in order) to take              */
+  unsigned pad1[31];
+  unsigned long long items, stale, edges, pushes, steps, splits;
+};
+
+struct WvParams {
+  const WvQuery *qs;
+  const unsigned *order;  /* largest first; NULL = 0..nq-1                     */
+  unsigned nq, groups, gsize; /* queries, groups of CTAs, CTAs of one        */
+  const WvArea *area;     /* [groups * gsize]                                  */
+  void *ws;
+  WvStat *st;
+  unsigned *grp;          /* a group's notes, two sets; cleared before a launch */
+  unsigned hops;          /* hops between two exchanges of a group             */
+  unsigned single_src;    /* overrides query 0's source when != ~0             */
+  unsigned filled;        /* the distances hold INF and the source already     */
+  unsigned low;           /* a frontier below this takes more far entries      */
+  unsigned high;          /* a frontier above this narrows the threshold step  */
+  unsigned long long timeout_ns;
+};
+
+#ifdef __cplusplus
+#include <cuda_runtime.h>
+#include <vector>
+
+struct WvEngine {
+  int device = -1;
+  bool flt = false;
+  int shape = -1;         /* kernel variant (wave.cu)                          */
+  unsigned nq = 0, groups = 0, gsize = 1, ctas = 0, req_gsize = 0;
+  unsigned *grp = nullptr;
+  WvQuery *qs = nullptr;
+  unsigned *order = nullptr;
+  WvArea *area = nullptr;
+  void *ws = nullptr;
+  WvStat *st = nullptr;
+  WvStat *st_host = nullptr; /* pinned                                         */
+  std::vector<WvQuery> qs_host;
+  size_t bytes = 0;
+};
+
+/* kernel variants: one CTA per query (256 or 1,024 threads), a group of CTAs,
+ * a group whose CTAs pool the edges of their entries */
+#define WV_CTA 0
+#define WV_WIDE 1
+#define WV_GROUP 2
+#define WV_POOL 3
+#define WV_LAST WV_POOL
+
+int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize,
+                    const std::vector<WvQuery> &qv, cudaStream_t st);
+void wv_engine_free(WvEngine &E);
+int wv_engine_reset(WvEngine &E, cudaStream_t st);
+int wv_engine_upload(WvEngine &E, cudaStream_t st);
+int wv_engine_enqueue(WvEngine &E, unsigned single_src, unsigned long long timeout_ns,
+                      cudaStream_t st, cudaEvent_t k0, cudaEvent_t k1);
+int wv_engine_status(const WvEngine &E, char *msg, size_t msg_len);
+#endif
+
+#endif /* ADDS_WAVE_INTERNAL_H_ */

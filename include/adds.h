@@ -115,7 +115,15 @@ typedef struct adds_opts {
                             the push.  Keeps a transposed copy of the graph
                             (8 B per edge, built on first use).  0 = auto
                             (on), < 0 = off, 1 = on                         */
-  int32_t reserved[2];
+  int32_t wave;          /* solve by a wave kernel (near-far lists, a CTA or a
+                            group of CTAs per query) instead of an engine,
+                            which takes over where its lists do not suffice:
+                            0 = auto (only where every knob of the schedule
+                            is automatic too), < 0 = no, 1 = a CTA of 256
+                            threads, 2 = a CTA of 1024, 3 = a CTA per SM
+                            (plain solves), 4 = a CTA per SM, pooling the
+                            edges of its entries (plain solves)              */
+  int32_t reserved[1];
 } adds_opts;
 
 /* Engines.  PHASE settles the buckets in bulk-synchronous phases (light
@@ -152,7 +160,8 @@ typedef struct adds_stats {
   int32_t delta_shift;      /* bucket shift at the end of the solve            */
   int32_t retries;          /* worklist regrowths needed                       */
   int32_t ctas;             /* persistent CTAs launched                        */
-  int32_t engine;           /* ADDS_ENGINE_ASYNC or ADDS_ENGINE_PHASE          */
+  int32_t engine;           /* ADDS_ENGINE_ASYNC or ADDS_ENGINE_PHASE: what ran,
+                               or what a wave kernel stood in for            */
   int32_t launches;         /* kernel launches per solve: async 2 (init, solver);
                                phase 1, or 5 with pull phases possible (phase,
                                pull, phase, pull, phase; unused ones return at

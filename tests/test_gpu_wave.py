@@ -1,0 +1,171 @@
+"""The wave kernels (one CTA or a group of CTAs per query, near-far lists)
+against the oracle, at the sizes and shapes where they can go wrong: frontiers
+that leave shared memory, rows around the length that is cut into pieces,
+groups of one CTA and of uneven size, thresholds of one unit and past every
+distance, equal paths, sums past INT32_MAX, and lists that overflow."""
+import numpy as np
+import pytest
+
+import adds_b200 as A
+from adds_b200 import graphs as G
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+CTA, WIDE, GROUP, POOL = 1, 2, 3, 4
+PIECE = 512  # edges of a long row per entry (wave_internal.h)
+
+
+def check(g, srcs, **kw):
+    dg = A.Graph.from_csr(g)
+    try:
+        st = None
+        for s in srcs:
+            d, st = dg.sssp(int(s), A.default_opts(timeout_ms=10000, **kw))
+            assert np.array_equal(d, O.dijkstra(g, int(s))[0]), (s, kw)
+        return st
+    finally:
+        dg.close()
+
+
+def star(rows, wtype=G.I32, seed=0):
+    """Vertex i has rows[i] edges to leaves of its own; the centres form a
+    path."""
+    src, dst, k = [], [], len(rows)
+    for i, r in enumerate(rows):
+        src += [i] * r + ([i] if i + 1 < len(rows) else [])
+        dst += list(range(k, k + r)) + ([i + 1] if i + 1 < len(rows) else [])
+        k += r
+    w = np.random.default_rng(seed).integers(1, 50, size=len(src))
+    return G.from_edges(k, src, dst, w.astype(np.float32) if wtype == G.F32 else w, wtype)
+
+
+@pytest.mark.parametrize("wave", [CTA, WIDE, GROUP, POOL])
+@pytest.mark.parametrize("wtype", [G.I32, G.F32])
+def test_graph_families(wave, wtype):
+    w = dict(wtype=wtype, w_lo=1, w_hi=100)
+    check(G.grid(97, 61, 0.02, 8, seed=3, **w), [0, 97 * 30 + 48], wave=wave)
+    check(G.erdos_renyi(3001, 8, seed=4, **w), [5, 2999], wave=wave)
+    r = G.rmat(13, 16, seed=5, **w)
+    assert r.degrees().max() > PIECE
+    check(r, [G.max_degree_vertex(r), 77], wave=wave)
+
+
+@pytest.mark.parametrize("wave", [CTA, WIDE, GROUP, POOL])
+def test_rows_around_the_piece_length(wave):
+    rows = [PIECE - 1, PIECE, PIECE + 1, 2 * PIECE, 2 * PIECE + 1, 7, 8, 9, 0, 5000]
+    for wtype in (G.I32, G.F32):
+        check(star(rows, wtype), [0, 4], wave=wave)
+
+
+@pytest.mark.parametrize("wave", [GROUP, POOL])
+@pytest.mark.parametrize("ctas", [1, 2, 7, 33, 148])
+def test_group_sizes(wave, ctas):
+    g = G.grid(80, 50, 0.02, 8, wtype=G.F32, w_lo=1.0, w_hi=100.0, seed=7)
+    st = check(g, [0, 2040], wave=wave, group_ctas=ctas)
+    assert st["ctas"] == ctas and st["retries"] == 0
+    check(G.rmat(12, 16, seed=8), [1], wave=wave, group_ctas=ctas)
+
+
+@pytest.mark.parametrize("wave", [CTA, WIDE, GROUP, POOL])
+@pytest.mark.parametrize("shift", [0, 3, 20, 31])
+def test_any_threshold_step(wave, shift):
+    check(G.grid(40, 40, 0.02, 8, wtype=G.F32, w_lo=1.0, w_hi=100.0, seed=9), [820], wave=wave,
+          delta_shift=shift)
+    check(G.erdos_renyi(900, 5, seed=10), [3], wave=wave, delta_shift=shift)
+
+
+@pytest.mark.parametrize("wave", [CTA, WIDE, GROUP, POOL])
+def test_special_weights_and_shapes(wave):
+    # equal paths everywhere: every weight 1, and zero-weight edges
+    side = 64
+    g = G.grid(side, side, 0.0, wtype=G.I32, w_lo=1, w_hi=1, seed=1)
+    check(g, [0, side * 32 + 32], wave=wave)
+    z = G.CSR(g.n, g.row, g.dst, np.zeros(g.m, np.uint32), G.I32)
+    check(z, [5], wave=wave)
+    # a chain, an isolated source, one vertex, self loops and double edges
+    n = 3000
+    check(G.from_edges(n, np.arange(n - 1), np.arange(1, n), np.full(n - 1, 7)), [0, n - 1], wave=wave)
+    check(G.from_edges(1, [], [], []), [0], wave=wave)
+    check(G.from_edges(3, [0, 0, 0, 1, 1], [0, 1, 1, 1, 2], [0, 9, 4, 1, 3]), [0], wave=wave)
+    # sums that reach INT32_MAX are never accepted
+    big = 0x7FFFFFFF
+    check(G.from_edges(5, [0, 1, 0, 3], [1, 2, 3, 4], [big - 1, 1, big, 0]), [0], wave=wave)
+    # infinite and very small float weights
+    w = np.array([np.inf, 1e-45, 3e38, 3e38], dtype=np.float32)
+    check(G.from_edges(5, [0, 0, 2, 3], [1, 2, 3, 4], w, G.F32), [0], wave=wave)
+
+
+def test_automatic_choice_and_overflow():
+    """Automatic knobs take a wave kernel; a frontier larger than its lists
+    sends the solve to the engine that grows, with the same distances."""
+    leaves = 300000
+    g = G.from_edges(leaves + 1, np.zeros(leaves, np.int64), np.arange(1, leaves + 1),
+                     np.full(leaves, 3))
+    dg = A.Graph.from_csr(g)
+    want = O.dijkstra(g, 0)[0]
+    d, st = dg.sssp(0, A.default_opts(timeout_ms=10000, wave=CTA))
+    assert st["retries"] == 1 and np.array_equal(d, want)
+    d, st = dg.sssp(0, A.default_opts(timeout_ms=10000, wave=CTA))  # remembered
+    assert st["retries"] == 0 and np.array_equal(d, want)
+    dg.close()
+    dg = A.Graph.from_csr(g)  # the same in the asynchronous form
+    for _ in range(3):
+        dg.sssp_async(0, A.default_opts(timeout_ms=10000, wave=CTA))
+    dg.sync()
+    assert np.array_equal(dg.last_dist(), want)
+    outs = [np.empty(g.n, np.uint32) for _ in range(3)]
+    dg.sssp_sources([0, 1, 0], outs)
+    assert np.array_equal(outs[0], want) and np.array_equal(outs[2], want)
+    dg.close()
+    for g in (G.grid(70, 70, 0.02, 8, wtype=G.F32, seed=2), G.grid(30, 20, 0.0, 8, seed=2),
+              G.rmat(12, 16, seed=2), G.erdos_renyi(2000, 8, seed=2)):
+        dg = A.Graph.from_csr(g)
+        d, st = dg.sssp(1)
+        assert np.array_equal(d, O.dijkstra(g, 1)[0])
+        auto = st["ctas"]
+        d, st = dg.sssp(1, A.default_opts(engine=2))
+        assert np.array_equal(d, O.dijkstra(g, 1)[0]) and st["ctas"] != auto
+        dg.close()
+
+
+@pytest.mark.parametrize("nq", [1, 5, 700])
+def test_sparse_batches(nq):
+    """Fewer and more queries than SMs, replayed, with new sources and new
+    weights between the runs."""
+    rng = np.random.default_rng(nq)
+    gs = [G.grid(20 + 7 * i, 15 + 5 * i, 0.02, 8, wtype=G.F32, seed=i) for i in range(5)]
+    dgs = [A.Graph.from_csr(g) for g in gs]
+    pick = [int(x) for x in rng.integers(0, len(gs), size=nq)]
+    b = A.Batch([dgs[p] for p in pick], [int(rng.integers(0, gs[p].n)) for p in pick])
+    for turn in range(3):
+        srcs = [int(rng.integers(0, gs[p].n)) for p in pick]
+        b.set_sources(srcs)
+        if turn == 2:
+            for i, g in enumerate(gs):
+                w = rng.uniform(0.5, 9, g.m).astype(np.float32)
+                gs[i] = G.CSR(g.n, g.row, g.dst, w.view(np.uint32), G.F32)
+                dgs[i].set_weights(w)
+        b.run()
+        b.run()
+        for q in range(0, nq, max(1, nq // 60)):
+            assert np.array_equal(b.dist(q), O.dijkstra(gs[pick[q]], srcs[q])[0]), (turn, q)
+    b.close()
+    for d in dgs:
+        d.close()
+
+
+def test_batch_overflow_moves_to_an_engine():
+    leaves = 300000
+    g = G.from_edges(leaves + 1, np.zeros(leaves, np.int64), np.arange(1, leaves + 1),
+                     np.full(leaves, 3))
+    r = G.grid(50, 50, 0.0, 8, wtype=G.I32, w_lo=1, w_hi=9, seed=1)
+    dg, dr = A.Graph.from_csr(g), A.Graph.from_csr(r)
+    b = A.Batch([dg, dr, dg] * 60, [0, 7, 1] * 60)
+    for _ in range(2):
+        b.run()
+        assert np.array_equal(b.dist(0), O.dijkstra(g, 0)[0])
+        assert np.array_equal(b.dist(1), O.dijkstra(r, 7)[0])
+        assert np.array_equal(b.dist(179), O.dijkstra(g, 1)[0])
+    b.close()
+    dg.close()
+    dr.close()
