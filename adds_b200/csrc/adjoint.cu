@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "../../include/adds.h"
@@ -35,7 +36,7 @@ int adds_batch_internal(adds_batch *b, cudaStream_t *st, unsigned *nq,
                         std::vector<adds_graph *> **ugraph, std::vector<unsigned> **qgid,
                         unsigned **dist_all, std::vector<size_t> **dist_off, void ***adj);
 void adds_graph_internal(const adds_graph *g, const unsigned **row, const uint2 **edges,
-                         uint32_t *n, uint64_t *m, int *device);
+                         uint32_t *n, uint64_t *m, unsigned *max_deg, int *device);
 
 #define NO_PRED 0xFFFFFFFFFFFFFFFFull
 #define NO_ROUND 0xFFFFFFFFu
@@ -46,12 +47,14 @@ struct AdjQ {
   const float *dist;
   const float *seed; /* dL/d dist */
   unsigned long long *pred;
-  float *lam;
-  unsigned *cnt;
-  unsigned *pend;
+  unsigned long long *lam; /* low half: lambda once it is known; until then
+                              what the children leave for each other       */
+  unsigned *kids; /* rows of at most 32 edges: which of them are tree edges;
+                     longer rows in the launch: how many are               */
   unsigned *round;
   unsigned n;
   unsigned src;
+  unsigned tile0; /* first tile of the query (TILE vertices each)          */
 };
 
 struct AdjG { /* one distinct graph and the queries that use it */
@@ -59,24 +62,45 @@ struct AdjG { /* one distinct graph and the queries that use it */
   float *grad;
   unsigned m;
   unsigned q_begin, q_end; /* into the query-index list */
+  unsigned tile0;          /* first tile of the graph (TILE edges each)    */
 };
 
 namespace adj {
 
-__global__ void k_init(const AdjQ *qs) {
-  const AdjQ &q = qs[blockIdx.y];
-  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < q.n; v += gridDim.x * blockDim.x) {
+constexpr unsigned TILE = 4096; /* vertices (or edges) a CTA takes            */
+
+/* The query (or graph) a CTA's tile belongs to and its first vertex (edge).
+ * One CTA per tile: a grid as long as the largest query for every query of a
+ * batch would be mostly empty CTAs (128 grids of side 64 to 512: 0.9 ms a
+ * kernel, whatever it did). */
+template <class T>
+__device__ __forceinline__ unsigned locate(const T *a, unsigned cnt, unsigned &first) {
+  unsigned lo = 0, hi = cnt - 1u;
+  while (lo < hi) {
+    const unsigned mid = (lo + hi + 1u) >> 1;
+    if (a[mid].tile0 <= blockIdx.x) lo = mid; else hi = mid - 1u;
+  }
+  first = (blockIdx.x - a[lo].tile0) * TILE;
+  return lo;
+}
+#define ADJ_TILE(q, v0, v1)                               \
+  unsigned v0;                                            \
+  const AdjQ &q = qs[locate(qs, nq, v0)];                 \
+  const unsigned v1 = min(q.n, v0 + TILE);
+
+__global__ void k_init(const AdjQ *qs, unsigned nq) {
+  ADJ_TILE(q, v0, v1)
+  for (unsigned v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
     q.pred[v] = NO_PRED;
-    q.cnt[v] = 0u;
-    q.lam[v] = 0.f;
-    q.round[v] = (v == q.src) ? 0u : NO_ROUND;
+    q.lam[v] = 0ull;
+    q.kids[v] = 0u;
   }
 }
 
 /* strict tight edges: d[u] < d[v] and fl(d[u] + w) == d[v] */
-__global__ void k_pred_strict(const AdjQ *qs) {
-  const AdjQ &q = qs[blockIdx.y];
-  for (unsigned u = blockIdx.x * blockDim.x + threadIdx.x; u < q.n; u += gridDim.x * blockDim.x) {
+__global__ void k_pred_strict(const AdjQ *qs, unsigned nq) {
+  ADJ_TILE(q, v0, v1)
+  for (unsigned u = v0 + threadIdx.x; u < v1; u += blockDim.x) {
     const float du = q.dist[u];
     if (__float_as_uint(du) == ADDS_INF_F32_BITSV) continue;
     const unsigned e1 = q.row[u + 1];
@@ -90,21 +114,40 @@ __global__ void k_pred_strict(const AdjQ *qs) {
   }
 }
 
-/* round 0 marks; count reached vertices left without a parent */
-__global__ void k_mark0(const AdjQ *qs, unsigned *orphans) {
-  const AdjQ &q = qs[blockIdx.y];
+/* Marks each vertex at its parent (MASK: the bit of its tree edge in the
+ * parent's row; else a count), and counts the reached vertices left without a
+ * parent. */
+template <bool MASK>
+__global__ void k_children(const AdjQ *qs, unsigned nq, unsigned *orphans) {
+  ADJ_TILE(q, v0, v1)
   unsigned c = 0;
-  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < q.n; v += gridDim.x * blockDim.x) {
-    if (q.pred[v] != NO_PRED) q.round[v] = 0u;
-    else if (v != q.src && __float_as_uint(q.dist[v]) != ADDS_INF_F32_BITSV) ++c;
+  for (unsigned v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+    const unsigned long long p = q.pred[v];
+    if (p != NO_PRED) {
+      const unsigned u = (unsigned)p;
+      if (MASK) atomicOr(&q.kids[u], 1u << ((unsigned)(p >> 32) - q.row[u]));
+      else atomicAdd(&q.kids[u], 1u);
+    } else if (v != q.src && __float_as_uint(q.dist[v]) != ADDS_INF_F32_BITSV) {
+      ++c;
+    }
   }
   if (c) atomicAdd(orphans, c);
 }
 
+/* Zero-gap ties only: rounds start from the vertices that have a parent, and
+ * the children are counted again afterwards. */
+__global__ void k_rounds_init(const AdjQ *qs, unsigned nq) {
+  ADJ_TILE(q, v0, v1)
+  for (unsigned v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+    q.round[v] = (v == q.src || q.pred[v] != NO_PRED) ? 0u : NO_ROUND;
+    q.kids[v] = 0u;
+  }
+}
+
 /* breadth-first round r over zero-gap tight edges */
-__global__ void k_pred_zero(const AdjQ *qs, unsigned r, unsigned *changed) {
-  const AdjQ &q = qs[blockIdx.y];
-  for (unsigned u = blockIdx.x * blockDim.x + threadIdx.x; u < q.n; u += gridDim.x * blockDim.x) {
+__global__ void k_pred_zero(const AdjQ *qs, unsigned nq, unsigned r, unsigned *changed) {
+  ADJ_TILE(q, v0, v1)
+  for (unsigned u = v0 + threadIdx.x; u < v1; u += blockDim.x) {
     if (q.round[u] >= r) continue; /* u must be in the tree before round r */
     const float du = q.dist[u];
     const unsigned e1 = q.row[u + 1];
@@ -122,65 +165,182 @@ __global__ void k_pred_zero(const AdjQ *qs, unsigned r, unsigned *changed) {
   }
 }
 
-__global__ void k_children(const AdjQ *qs) {
-  const AdjQ &q = qs[blockIdx.y];
-  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < q.n; v += gridDim.x * blockDim.x) {
-    const unsigned long long p = q.pred[v];
-    if (p != NO_PRED) atomicAdd(&q.cnt[(unsigned)p], 1u);
+__device__ __forceinline__ float lam_of(const AdjQ &q, unsigned v) {
+  return __uint_as_float((unsigned)__ldcg(q.lam + v));
+}
+
+/* acc (the seed of x) plus lambda of x's children, in x's CSR edge order */
+template <bool MASK>
+__device__ __forceinline__ float gather_lambda(const AdjQ &q, unsigned x, unsigned kids, float acc) {
+  const unsigned r0 = __ldg(q.row + x);
+  if (MASK) {
+    for (; kids; kids &= kids - 1u)
+      acc = __fadd_rn(acc, lam_of(q, __ldg(&q.edges[r0 + (unsigned)__ffs(kids) - 1u].x)));
+    return acc;
   }
-}
-
-__global__ void k_copy_pend(const AdjQ *qs) {
-  const AdjQ &q = qs[blockIdx.y];
-  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < q.n; v += gridDim.x * blockDim.x)
-    q.pend[v] = q.cnt[v];
-}
-
-/* lambda of x from its seed and its children, in x's CSR edge order */
-__device__ __forceinline__ float gather_lambda(const AdjQ &q, unsigned x) {
-  float acc = q.seed ? __ldcg(q.seed + x) : 0.f;
-  const unsigned e1 = q.row[x + 1];
-  for (unsigned e = q.row[x]; e < e1; ++e) {
+  const unsigned e1 = __ldg(q.row + x + 1);
+  for (unsigned e = r0; e < e1; ++e) {
     const unsigned v = q.edges[e].x;
-    const unsigned long long p = __ldcg(&q.pred[v]);
-    if ((unsigned)(p >> 32) == e && p != NO_PRED) acc = __fadd_rn(acc, __ldcg(q.lam + v));
+    const unsigned long long p = __ldg(&q.pred[v]);
+    if ((unsigned)(p >> 32) == e && p != NO_PRED) acc = __fadd_rn(acc, lam_of(q, v));
   }
   return acc;
 }
 
-/* every leaf of the tree starts a walk; the last child to finish carries
- * on with its parent */
-__global__ void k_walk(const AdjQ *qs) {
-  const AdjQ &q = qs[blockIdx.y];
-  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < q.n; v += gridDim.x * blockDim.x) {
-    if (q.cnt[v] != 0u) continue;
-    if (__float_as_uint(q.dist[v]) == ADDS_INF_F32_BITSV) continue;
-    unsigned x = v;
-    for (unsigned hops = 0; hops <= q.n; ++hops) {
-      const float l = gather_lambda(q, x);
-      __stcg(q.lam + x, l);
-      const unsigned long long p = __ldcg(&q.pred[x]);
-      if (p == NO_PRED) break; /* the source (or an unreached root) */
-      const unsigned parent = (unsigned)p;
-      __threadfence();
-      if (atomicSub(&q.pend[parent], 1u) != 1u) break; /* siblings still running */
-      __threadfence();
-      x = parent;
+/* A walk handed from the first launch of walks to the second. */
+struct __align__(16) Walk {
+  unsigned q, x;
+  float acc; /* lambda of x, complete */
+  unsigned pad;
+};
+
+/* Every leaf of the tree starts a walk to the root; the last child of a vertex
+ * to finish carries on with it.  An only child carries on without asking; of
+ * two, the first leaves its lambda in the parent's word and the second takes
+ * it with the same exchange; of more, each counts itself there and the last
+ * reads the others'.  So a step is one round trip for what the parent needs and
+ * mostly at most one atomic, with no fence; lanes that do need fences wait until
+ * SLOW of the warp do, since the others would wait with them.
+ *
+ * Bound by those round trips and by the lanes that take part: walks are a few
+ * steps long on average and hundreds at worst.  FIRST: a warp takes the leaves
+ * of neighbouring vertices, a lane whose walk has ended takes the next leaf,
+ * and once the leaves are out and at most HAND walks go on these are handed to
+ * a second launch: long walks would keep a CTA's place on the SM for a lane or
+ * two (a third of the warps resident, 17 lanes active).  That launch gives each
+ * warp HAND walks at a time.
+ * 128 grids x 16 sources: 37 ms when the lanes of a warp waited for the longest
+ * of their 32 walks; 15 with lanes refilled but a fence, a count and a read of
+ * every child at each vertex; 9.0 with exchanges instead; 3.8 + 3.1 now. */
+constexpr unsigned SLOW = 8u, HAND = 4u;
+template <bool MASK, bool FIRST, bool HANDS>
+__global__ void __launch_bounds__(512, 2) k_walk(const AdjQ *qs, unsigned nq, Walk *hand,
+                                                 unsigned *ctr) {
+  /* ctr: walks handed over, walks taken up */
+  const unsigned lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  __shared__ unsigned short list[FIRST ? TILE : 1u];
+  unsigned t0 = 0, qi = 0, end = 0, next = 0, v0 = 0;
+  const unsigned own = TILE / (blockDim.x / 32u), at = FIRST ? (threadIdx.x >> 5) * own : 0u;
+  unsigned short *const leaf = list + at;
+  if (FIRST) qi = locate(qs, nq, t0);
+  AdjQ q = qs[qi];
+  if (FIRST) { /* the leaves among the warp's vertices */
+    v0 = t0 + at;
+    const unsigned v1 = min(q.n, v0 + own);
+#pragma unroll 4
+    for (unsigned i = v0; i < v1; i += 32u) {
+      const unsigned v = i + lane;
+      const bool is = v < v1 && __ldg(q.kids + v) == 0u &&
+                      __float_as_uint(__ldg(q.dist + v)) != ADDS_INF_F32_BITSV;
+      const unsigned b = __ballot_sync(0xFFFFFFFFu, is);
+      if (is) leaf[end + __popc(b & lt)] = (unsigned short)(v - v0);
+      end += __popc(b);
+    }
+    __syncwarp();
+  } else {
+    end = ctr[0];
+  }
+  bool busy = false;
+  unsigned x = 0;
+  float acc = 0.f;                /* lambda of x, complete */
+  unsigned long long p = NO_PRED; /* pred of x */
+  unsigned kids = 0, k = 0;       /* children of x (k: 1, 2 or more)            */
+  float seed = 0.f;
+  while (next < end || __any_sync(0xFFFFFFFFu, busy)) {
+    const unsigned idle = __ballot_sync(0xFFFFFFFFu, !busy);
+    bool fresh = false; /* its first loads overlap the other lanes' step */
+    if (FIRST) { /* idle lanes take the next leaves */
+      const unsigned i = next + __popc(idle & lt);
+      if (!busy && i < end) {
+        busy = fresh = true;
+        x = v0 + leaf[i];
+        k = 0u;
+        acc = q.seed ? __ldg(q.seed + x) : 0.f;
+        p = __ldg(&q.pred[x]);
+      }
+      next += __popc(idle);
+    } else if (next < end && (idle & ((1u << HAND) - 1u))) { /* or the next walks */
+      unsigned i = end;
+      if (!busy && lane < HAND) i = atomicAdd(ctr + 1, 1u);
+      if (i < end) {
+        const Walk w = hand[i];
+        busy = fresh = true;
+        q = qs[w.q];
+        x = w.x;
+        k = 0u;
+        acc = w.acc;
+        p = __ldg(&q.pred[x]);
+      }
+      /* the counter only rises: once past the end nothing is left */
+      if (__any_sync(0xFFFFFFFFu, !busy && lane < HAND)) next = end;
+    }
+    if (busy && !fresh && k <= 2u) {
+      __stcg(reinterpret_cast<unsigned *>(q.lam + x), __float_as_uint(acc));
+      busy = p != NO_PRED; /* else the source (or an unreached root) */
+      if (busy) {
+        const unsigned e = (unsigned)(p >> 32);
+        x = (unsigned)p; /* the parent; acc is its child's until it is complete */
+        kids = __ldg(q.kids + x);
+        const unsigned r0 = MASK ? __ldg(q.row + x) : 0u;
+        seed = q.seed ? __ldg(q.seed + x) : 0.f;
+        p = __ldg(&q.pred[x]);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(q.lam + x));
+        k = MASK ? (unsigned)__popc(kids) : kids;
+        if (k == 1u) {
+          acc = __fadd_rn(seed, acc);
+        } else if (MASK && k == 2u) {
+          const unsigned long long old =
+              atomicExch(q.lam + x, (1ull << 32) | __float_as_uint(acc));
+          busy = (old >> 32) != 0ull; /* else the sibling still runs */
+          const float other = __uint_as_float((unsigned)old);
+          const bool mine = (kids & (0u - kids)) == 1u << (e - r0); /* this child's edge first */
+          acc = __fadd_rn(__fadd_rn(seed, mine ? acc : other), mine ? other : acc);
+        } else {
+          k = 3u; /* waits for the slow way below */
+        }
+      }
+    }
+    const unsigned slow = __ballot_sync(0xFFFFFFFFu, busy && k > 2u);
+    const unsigned going = __ballot_sync(0xFFFFFFFFu, busy);
+    const bool last = HANDS && next >= end && __popc(going) <= (int)HAND;
+    if (slow != 0u && (last || __popc(slow) >= (int)(FIRST ? SLOW : 1u) || slow == going)) {
+      if (busy && k > 2u) {
+        const unsigned all = MASK ? (unsigned)__popc(kids) : kids;
+        /* lambda of the child, before it counts as finished; the siblings'
+         * counts, before their lambdas are read */
+        unsigned long long old;
+        asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], %2;"
+                     : "=l"(old) : "l"(q.lam + x), "l"(1ull << 32) : "memory");
+        busy = (unsigned)(old >> 32) + 1u == all; /* else siblings still run */
+        if (busy) acc = gather_lambda<MASK>(q, x, kids, seed);
+        k = 1u;
+      }
+    }
+    if (last) {
+      const unsigned b = __ballot_sync(0xFFFFFFFFu, busy);
+      unsigned i = 0;
+      if (lane == 0 && b) i = atomicAdd(ctr, (unsigned)__popc(b));
+      i = __shfl_sync(0xFFFFFFFFu, i, 0);
+      if (busy) hand[i + __popc(b & lt)] = Walk{qi, x, acc, 0u};
+      break;
     }
   }
 }
 
 /* grad[e] (+)= sum over the graph's queries, in query order, of lambda at
  * dst(e) when e is that vertex's tree edge */
-__global__ void k_grad(const AdjG *gs, const AdjQ *qs, const unsigned *qidx, int accumulate) {
-  const AdjG &g = gs[blockIdx.y];
-  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < g.m; e += gridDim.x * blockDim.x) {
+__global__ void k_grad(const AdjG *gs, unsigned ng, const AdjQ *qs, const unsigned *qidx,
+                       int accumulate) {
+  unsigned e0;
+  const AdjG &g = gs[locate(gs, ng, e0)];
+  const unsigned e1 = (unsigned)min((unsigned long long)g.m, (unsigned long long)e0 + TILE);
+  for (unsigned e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
     const unsigned v = g.edges[e].x;
     float acc = 0.f;
     for (unsigned i = g.q_begin; i < g.q_end; ++i) {
       const AdjQ &q = qs[qidx[i]];
       const unsigned long long p = q.pred[v];
-      if (p != NO_PRED && (unsigned)(p >> 32) == e) acc = __fadd_rn(acc, q.lam[v]);
+      if (p != NO_PRED && (unsigned)(p >> 32) == e) acc = __fadd_rn(acc, __uint_as_float((unsigned)q.lam[v]));
     }
     g.grad[e] = accumulate ? __fadd_rn(g.grad[e], acc) : acc;
   }
@@ -196,6 +356,8 @@ struct AdjScratch {
   AdjG *d_gs = nullptr;
   unsigned *d_qidx = nullptr;
   unsigned *d_flag = nullptr;
+  void *d_hand = nullptr;
+  size_t cap_hand = 0;
   size_t nq = 0, ng = 0;
 };
 
@@ -207,6 +369,7 @@ void adds_adjoint_free(void *p) {
   if (s->d_gs) cudaFree(s->d_gs);
   if (s->d_qidx) cudaFree(s->d_qidx);
   if (s->d_flag) cudaFree(s->d_flag);
+  if (s->d_hand) cudaFree(s->d_hand);
   delete s;
 }
 
@@ -223,7 +386,8 @@ static int adj_fail(cudaError_t e) {
 /* Core: queries (row, edges, n, src, dist, seed) + graphs (edges, m, grad,
  * query list) -> gradient. */
 static int run_adjoint(AdjScratch *S, std::vector<AdjQ> &qh, std::vector<AdjG> &gh,
-                       const std::vector<unsigned> &qidx, int accumulate, cudaStream_t st) {
+                       const std::vector<unsigned> &qidx, unsigned max_deg, int accumulate,
+                       cudaStream_t st) {
   size_t need = 0;
   unsigned max_n = 0;
   for (auto &q : qh) {
@@ -251,55 +415,82 @@ static int run_adjoint(AdjScratch *S, std::vector<AdjQ> &qh, std::vector<AdjG> &
     CKA(cudaMalloc(&S->d_qidx, qidx.size() * sizeof(unsigned)));
     S->ng = gh.size();
   }
-  if (!S->d_flag) CKA(cudaMalloc(&S->d_flag, 8));
-  /* carve: pred u64 | lam f32 | cnt | pend | round */
+  if (!S->d_flag) CKA(cudaMalloc(&S->d_flag, 16));
+  /* carve: pred u64 | lam u64 | kids | round */
   unsigned long long *pred = (unsigned long long *)S->mem;
-  float *lam = (float *)(pred + need);
-  unsigned *cnt = (unsigned *)(lam + need);
-  unsigned *pend = cnt + need;
-  unsigned *round = pend + need;
+  unsigned long long *lam = pred + need;
+  unsigned *kids = (unsigned *)(lam + need);
+  unsigned *round = kids + need;
   size_t off = 0;
+  unsigned long long tiles = 0, etiles = 0;
   for (auto &q : qh) {
     q.pred = pred + off;
     q.lam = lam + off;
-    q.cnt = cnt + off;
-    q.pend = pend + off;
+    q.kids = kids + off;
     q.round = round + off;
     off += ((size_t)q.n + 31) & ~(size_t)31;
+    q.tile0 = (unsigned)tiles;
+    tiles += (q.n + adj::TILE - 1u) / adj::TILE;
   }
+  for (auto &g : gh) {
+    g.tile0 = (unsigned)etiles;
+    etiles += ((unsigned long long)g.m + adj::TILE - 1u) / adj::TILE;
+  }
+  /* HAND walks of each of a tile's 4 warps */
+  const size_t hands = (size_t)tiles * 4u * adj::HAND;
+  if (hands > S->cap_hand) {
+    if (S->d_hand) cudaFree(S->d_hand);
+    S->d_hand = nullptr;
+    S->cap_hand = 0;
+    CKA(cudaMalloc(&S->d_hand, hands * sizeof(adj::Walk)));
+    S->cap_hand = hands;
+  }
+  if (tiles > 0x7FFFFFFFull || etiles > 0x7FFFFFFFull) return ADDS_ERR_UNSUPPORTED;
   CKA(cudaMemcpyAsync(S->d_qs, qh.data(), qh.size() * sizeof(AdjQ), cudaMemcpyHostToDevice, st));
   CKA(cudaMemcpyAsync(S->d_gs, gh.data(), gh.size() * sizeof(AdjG), cudaMemcpyHostToDevice, st));
   CKA(cudaMemcpyAsync(S->d_qidx, qidx.data(), qidx.size() * sizeof(unsigned),
                       cudaMemcpyHostToDevice, st));
-  unsigned bx = (max_n + 255u) / 256u;
-  if (bx > 592u) bx = 592u;
-  if (bx == 0u) bx = 1u;
-  const dim3 grid(bx, (unsigned)qh.size());
-  adj::k_init<<<grid, 256, 0, st>>>(S->d_qs);
-  adj::k_pred_strict<<<grid, 256, 0, st>>>(S->d_qs);
+  const unsigned nq = (unsigned)qh.size(), ng = (unsigned)gh.size(), T = (unsigned)tiles;
+  auto children = [&] {
+    if (max_deg <= 32u) adj::k_children<true><<<T, 256, 0, st>>>(S->d_qs, nq, S->d_flag);
+    else adj::k_children<false><<<T, 256, 0, st>>>(S->d_qs, nq, S->d_flag);
+  };
+  adj::k_init<<<T, 256, 0, st>>>(S->d_qs, nq);
+  adj::k_pred_strict<<<T, 256, 0, st>>>(S->d_qs, nq);
   CKA(cudaMemsetAsync(S->d_flag, 0, 8, st));
-  adj::k_mark0<<<grid, 256, 0, st>>>(S->d_qs, S->d_flag);
+  children();
   unsigned orphans = 0;
   CKA(cudaMemcpyAsync(&orphans, S->d_flag, 4, cudaMemcpyDeviceToHost, st));
   CKA(cudaStreamSynchronize(st));
-  for (unsigned r = 1; orphans && r <= max_n; ++r) { /* zero-gap ties only */
-    unsigned changed = 0;
-    CKA(cudaMemsetAsync(S->d_flag, 0, 4, st));
-    adj::k_pred_zero<<<grid, 256, 0, st>>>(S->d_qs, r, S->d_flag);
-    CKA(cudaMemcpyAsync(&changed, S->d_flag, 4, cudaMemcpyDeviceToHost, st));
-    CKA(cudaStreamSynchronize(st));
-    if (!changed) break;
+  if (orphans) { /* zero-gap ties */
+    adj::k_rounds_init<<<T, 256, 0, st>>>(S->d_qs, nq);
+    for (unsigned r = 1; r <= max_n; ++r) {
+      unsigned changed = 0;
+      CKA(cudaMemsetAsync(S->d_flag, 0, 4, st));
+      adj::k_pred_zero<<<T, 256, 0, st>>>(S->d_qs, nq, r, S->d_flag);
+      CKA(cudaMemcpyAsync(&changed, S->d_flag, 4, cudaMemcpyDeviceToHost, st));
+      CKA(cudaStreamSynchronize(st));
+      if (!changed) break;
+    }
+    children();
   }
-  adj::k_children<<<grid, 256, 0, st>>>(S->d_qs);
-  adj::k_copy_pend<<<grid, 256, 0, st>>>(S->d_qs);
-  adj::k_walk<<<grid, 256, 0, st>>>(S->d_qs);
-  unsigned max_m = 0;
-  for (auto &g : gh)
-    if (g.m > max_m) max_m = g.m;
-  unsigned gx = (max_m + 255u) / 256u;
-  if (gx > 592u) gx = 592u;
-  if (gx == 0u) gx = 1u;
-  adj::k_grad<<<dim3(gx, (unsigned)gh.size()), 256, 0, st>>>(S->d_gs, S->d_qs, S->d_qidx, accumulate);
+  if (T >= 8u * 148u) {
+    adj::Walk *hand = (adj::Walk *)S->d_hand;
+    unsigned *ctr = S->d_flag + 2;
+    CKA(cudaMemsetAsync(ctr, 0, 8, st));
+    if (max_deg <= 32u) {
+      adj::k_walk<true, true, true><<<T, 128, 0, st>>>(S->d_qs, nq, hand, ctr);
+      adj::k_walk<true, false, false><<<148 * 12, 128, 0, st>>>(S->d_qs, nq, hand, ctr);
+    } else {
+      adj::k_walk<false, true, true><<<T, 128, 0, st>>>(S->d_qs, nq, hand, ctr);
+      adj::k_walk<false, false, false><<<148 * 12, 128, 0, st>>>(S->d_qs, nq, hand, ctr);
+    }
+  } else { /* too few tiles to fill the SMs: nothing to make room for */
+    if (max_deg <= 32u) adj::k_walk<true, true, false><<<T, 512, 0, st>>>(S->d_qs, nq, nullptr, nullptr);
+    else adj::k_walk<false, true, false><<<T, 512, 0, st>>>(S->d_qs, nq, nullptr, nullptr);
+  }
+  if (etiles)
+    adj::k_grad<<<(unsigned)etiles, 256, 0, st>>>(S->d_gs, ng, S->d_qs, S->d_qidx, accumulate);
   CKA(cudaGetLastError());
   CKA(cudaStreamSynchronize(st));
   return ADDS_OK;
@@ -321,12 +512,13 @@ extern "C" int adds_batch_backward(adds_batch *b, const float *const *grad_dist,
   const uint2 *edges;
   uint32_t n;
   uint64_t m;
+  unsigned deg, max_deg = 0;
   int dev;
-  adds_graph_internal((*qgraph)[0], &row, &edges, &n, &m, &dev);
+  adds_graph_internal((*qgraph)[0], &row, &edges, &n, &m, &deg, &dev);
   CKA(cudaSetDevice(dev));
   std::vector<AdjQ> qh(nq);
   for (unsigned i = 0; i < nq; ++i) {
-    adds_graph_internal((*qgraph)[i], &row, &edges, &n, &m, &dev);
+    adds_graph_internal((*qgraph)[i], &row, &edges, &n, &m, &deg, &dev);
     AdjQ q;
     memset(&q, 0, sizeof q);
     q.row = row;
@@ -340,9 +532,10 @@ extern "C" int adds_batch_backward(adds_batch *b, const float *const *grad_dist,
   std::vector<AdjG> gh(ugraph->size());
   std::vector<unsigned> qidx;
   for (size_t gi = 0; gi < ugraph->size(); ++gi) {
-    adds_graph_internal((*ugraph)[gi], &row, &edges, &n, &m, &dev);
+    adds_graph_internal((*ugraph)[gi], &row, &edges, &n, &m, &deg, &dev);
     if (!grad_w[gi]) return ADDS_ERR_INVALID;
     AdjG g;
+    max_deg = std::max(max_deg, deg);
     g.edges = edges;
     g.m = (unsigned)m;
     g.grad = grad_w[gi];
@@ -353,7 +546,7 @@ extern "C" int adds_batch_backward(adds_batch *b, const float *const *grad_dist,
     gh[gi] = g;
   }
   if (!*adjp) *adjp = new AdjScratch();
-  return run_adjoint((AdjScratch *)*adjp, qh, gh, qidx, 1, st);
+  return run_adjoint((AdjScratch *)*adjp, qh, gh, qidx, max_deg, 1, st);
 }
 
 extern "C" int adds_sssp_backward(adds_graph *g, uint32_t ns, const uint32_t *srcs, const float *dist,
@@ -363,8 +556,9 @@ extern "C" int adds_sssp_backward(adds_graph *g, uint32_t ns, const uint32_t *sr
   const uint2 *edges;
   uint32_t n;
   uint64_t m;
+  unsigned deg;
   int dev;
-  adds_graph_internal(g, &row, &edges, &n, &m, &dev);
+  adds_graph_internal(g, &row, &edges, &n, &m, &deg, &dev);
   for (uint32_t i = 0; i < ns; ++i)
     if (srcs[i] >= n) return ADDS_ERR_INVALID;
   CKA(cudaSetDevice(dev));
@@ -390,11 +584,12 @@ extern "C" int adds_sssp_backward(adds_graph *g, uint32_t ns, const uint32_t *sr
   gh[0].q_begin = 0;
   gh[0].q_end = ns;
   AdjScratch S;
-  const int rc = run_adjoint(&S, qh, gh, qidx, 0, st);
+  const int rc = run_adjoint(&S, qh, gh, qidx, deg, 0, st);
   if (S.mem) cudaFree(S.mem);
   if (S.d_qs) cudaFree(S.d_qs);
   if (S.d_gs) cudaFree(S.d_gs);
   if (S.d_qidx) cudaFree(S.d_qidx);
   if (S.d_flag) cudaFree(S.d_flag);
+  if (S.d_hand) cudaFree(S.d_hand);
   return rc;
 }

@@ -2282,7 +2282,8 @@ int adds_batch_internal(adds_batch *b, cudaStream_t *st, unsigned *nq,
   return ADDS_OK;
 }
 void adds_graph_internal(const adds_graph *g, const unsigned **row, const uint2 **edges,
-                         uint32_t *n, uint64_t *m, int *device) {
+                         uint32_t *n, uint64_t *m, unsigned *max_deg, int *device) {
+  *max_deg = g->max_deg;
   *row = g->row;
   *edges = g->edges;
   *n = g->n;

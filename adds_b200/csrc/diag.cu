@@ -19,7 +19,7 @@
 #include "adds_internal.h"
 
 void adds_graph_internal(const adds_graph *g, const unsigned **row, const uint2 **edges,
-                         uint32_t *n, uint64_t *m, int *device);
+                         uint32_t *n, uint64_t *m, unsigned *max_deg, int *device);
 void adds_set_last_error(const char *msg);
 
 namespace {
@@ -80,8 +80,9 @@ extern "C" int adds_diag_relax_pass(adds_graph *g, uint32_t src, double ms_out[4
   const uint2 *edges;
   uint32_t n;
   uint64_t m;
+  unsigned max_deg;
   int dev;
-  adds_graph_internal(g, &row, &edges, &n, &m, &dev);
+  adds_graph_internal(g, &row, &edges, &n, &m, &max_deg, &dev);
   if (src >= n) return ADDS_ERR_INVALID;
   if (cudaSetDevice(dev) != cudaSuccess) return ADDS_ERR_CUDA;
   /* the final distances of one solve from src */
