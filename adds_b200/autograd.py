@@ -22,11 +22,15 @@ from . import Batch
 class _SSSP(torch.autograd.Function):
     @staticmethod
     def forward(ctx, batch: Batch, graphs: list, *weights):
-        for g, w in zip(graphs, weights):
-            g.set_weights(w.detach().contiguous().data_ptr())
-        batch.run()
         off, tot = batch.layout()
         flat = torch.zeros(int(tot), dtype=torch.float32, device=weights[0].device)
+        held = [w.detach().contiguous() for w in weights]
+        # the graphs and the batch work on streams of their own: the weights
+        # must have been computed, and the zeros written, before they start
+        torch.cuda.current_stream(flat.device).synchronize()
+        for g, w in zip(graphs, held):
+            g.set_weights(w.data_ptr())
+        batch.run()
         batch.dist_all(flat.data_ptr())
         ctx.batch = batch
         ctx.off = off
