@@ -1338,58 +1338,41 @@ static int graph_phase_engine(adds_graph *g, const Knobs &k, int shift, float sc
   return rc;
 }
 
-/* Pieces of the rows that one warp of a wave kernel should not relax alone:
- * counted per row, numbered by a scan, written out.  Depends on the rows
- * only, so it is made once per graph. */
-__global__ void k_piece_count(const unsigned *row, uint32_t n, unsigned *cnt) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x) {
-    const unsigned deg = v < n ? row[v + 1] - row[v] : 0u;
-    cnt[v] = deg > WV_PIECE ? (deg + WV_PIECE - 1u) / WV_PIECE : 0u;
-  }
-}
-__global__ void k_piece_fill(const unsigned *row, uint32_t n, const unsigned *first, uint4 *piece) {
+/* Pieces of the rows that one warp of a wave kernel should not relax alone,
+ * numbered in whatever order the counter gives.  Depends on the rows only, so
+ * it is made once per graph. */
+__global__ void k_pieces(const unsigned *row, uint32_t n, unsigned *cnt, unsigned *first,
+                         uint4 *piece) {
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    const unsigned r1 = row[v + 1], c1 = first[v + 1];
-    unsigned e = row[v];
-    for (unsigned c = first[v]; c < c1; ++c, e += WV_PIECE)
-      piece[c] = make_uint4(v, e, min(WV_PIECE, r1 - e), 0u);
+    const unsigned r0 = row[v], deg = row[v + 1] - r0;
+    if (deg <= WV_PIECE) continue;
+    const unsigned k = (deg + WV_PIECE - 1u) / WV_PIECE, c = atomicAdd(cnt, k);
+    first[v] = c;
+    for (unsigned j = 0; j < k; ++j)
+      piece[c + j] = make_uint4(v, r0 + j * WV_PIECE, min(WV_PIECE, deg - j * WV_PIECE), 0u);
   }
 }
 
 static int graph_pieces(adds_graph *g) {
   if (g->wpiece || g->max_deg <= WV_PIECE) return ADDS_OK;
-  const size_t n = g->n;
-  unsigned *cnt = nullptr;
-  void *tmp = nullptr;
-  size_t tb = 0;
-  unsigned total = 0;
+  /* a row longer than a piece has fewer than twice as many as its edges fill */
+  const size_t cap = 2 * (g->m / WV_PIECE) + 1;
   cudaError_t e = cudaSuccess;
-  if (!g->wfirst) e = cudaMalloc(&g->wfirst, (n + 1) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&cnt, (n + 1) * 4);
+  if (!g->wfirst) e = cudaMalloc(&g->wfirst, ((size_t)g->n + 1) * 4);
+  if (e == cudaSuccess) e = cudaMalloc(&g->wpiece, cap * sizeof(uint4));
+  unsigned *cnt = g->wfirst ? g->wfirst + g->n : nullptr;
+  if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, 4, g->stream);
   if (e == cudaSuccess) {
-    k_piece_count<<<592, 256, 0, g->stream>>>(g->row, g->n, cnt);
-    e = cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, g->wfirst, (int)(n + 1), g->stream);
-  }
-  if (e == cudaSuccess) e = cudaMalloc(&tmp, tb ? tb : 16);
-  if (e == cudaSuccess)
-    e = cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, g->wfirst, (int)(n + 1), g->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&total, g->wfirst + n, 4, cudaMemcpyDeviceToHost, g->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  if (e == cudaSuccess) e = cudaMalloc(&g->wpiece, ((size_t)total + 1) * sizeof(uint4));
-  if (e == cudaSuccess) {
-    k_piece_fill<<<592, 256, 0, g->stream>>>(g->row, g->n, g->wfirst, g->wpiece);
+    k_pieces<<<592, 256, 0, g->stream>>>(g->row, g->n, cnt, g->wfirst, g->wpiece);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  if (cnt) cudaFree(cnt);
-  if (tmp) cudaFree(tmp);
   if (e != cudaSuccess) {
     if (g->wpiece) cudaFree(g->wpiece);
     g->wpiece = nullptr;
     return cuda_fail(e, "pieces of long rows");
   }
-  g->bytes += (n + 1) * 4 + (size_t)total * sizeof(uint4);
+  g->bytes += ((size_t)g->n + 1) * 4 + cap * sizeof(uint4);
   return ADDS_OK;
 }
 

@@ -49,6 +49,7 @@
 #define PH_ERR_MAPPING 4u
 #define PH_ERR_INPUT 5u    /* caller's arrays failed validation (no-alloc path);
                               err_where holds the failed checks            */
+#define PH_ERR_SOLVED 6u   /* no-alloc path: solved before this engine's launch */
 
 /* Read-only per-query descriptor. */
 struct PhQuery {

@@ -838,7 +838,7 @@ static unsigned wv_low(int shape) {
 #undef X
   return 0;
 }
-static unsigned wv_near(int shape) {
+unsigned wv_near(int shape) {
 #define X(s, b, ns, m, g, pl, lo) if (shape == s) return ns;
   WV_SHAPES(X)
 #undef X
@@ -881,12 +881,7 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
   int sms = 0, bps = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
     return -5;
-  cudaError_t e = cudaErrorInvalidValue;
-#define X(s, b, ns, m, g, pl, lo) \
-  if (shape == s)         \
-    e = flt ? resident<true, b, ns, m, g, pl>(&bps) : resident<false, b, ns, m, g, pl>(&bps);
-  WV_SHAPES(X)
-#undef X
+  const cudaError_t e = wv_prepare(flt, shape, &bps);
   if (e != cudaSuccess || bps < 1) {
     cudaGetLastError();
     return -9;
@@ -970,6 +965,38 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
   return rc ? rc : wv_engine_reset(E, st);
 }
 
+void wv_schedule(WvParams &P, int shape, unsigned n, bool pieces) {
+  P.low = wv_low(shape) * P.gsize;
+  P.high = wv_block(shape) * P.gsize * 4u;
+  /* Hops on a CTA's own entries between two exchanges.  Roads: 8 (a 4096^2
+   * grid 18.3 ms, against 19.3 at 4 and 33 at 1, where the exchanges cost more
+   * than the hops).  Pooled: 1, since the neighbours of an entry are anywhere
+   * and hops on stale distances relax too much (R-MAT 16 0.38 ms, 0.60 at 8),
+   * but 8 on graphs so small that the few hops are all there is (20,000
+   * vertices 0.20 ms, 0.27 at 1). */
+  P.hops = shape == WV_GROUP || (n < 32768u && !pieces) ? 8u : 1u;
+}
+
+cudaError_t wv_prepare(bool flt, int shape, int *bps) {
+  using namespace adds_wave;
+#define X(s, b, ns, m, g, pl, lo) \
+  if (shape == s)                 \
+    return flt ? resident<true, b, ns, m, g, pl>(bps) : resident<false, b, ns, m, g, pl>(bps);
+  WV_SHAPES(X)
+#undef X
+  return cudaErrorInvalidValue;
+}
+
+cudaError_t wv_launch(const WvParams &P, bool flt, int shape, cudaStream_t st) {
+  using namespace adds_wave;
+#define X(s, b, ns, m, g, pl, lo) \
+  if (shape == s)                 \
+    return flt ? launch<true, b, ns, m, g, pl>(P, st) : launch<false, b, ns, m, g, pl>(P, st);
+  WV_SHAPES(X)
+#undef X
+  return cudaErrorInvalidValue;
+}
+
 int wv_engine_enqueue(WvEngine &E, unsigned single_src, unsigned long long timeout_ns,
                       cudaStream_t st, cudaEvent_t k0, cudaEvent_t k1) {
   using namespace adds_wave;
@@ -993,15 +1020,7 @@ int wv_engine_enqueue(WvEngine &E, unsigned single_src, unsigned long long timeo
   P.grp = E.grp;
   P.single_src = single_src;
   P.timeout_ns = timeout_ns;
-  P.low = wv_low(E.shape) * E.gsize;
-  P.high = wv_block(E.shape) * E.gsize * 4u;
-  /* Hops on a CTA's own entries between two exchanges.  Roads: 8 (a 4096^2
-   * grid 18.3 ms, against 19.3 at 4 and 33 at 1, where the exchanges cost more
-   * than the hops).  Pooled: 1, since the neighbours of an entry are anywhere
-   * and hops on stale distances relax too much (R-MAT 16 0.38 ms, 0.60 at 8),
-   * but 8 on graphs so small that the few hops are all there is (20,000
-   * vertices 0.20 ms, 0.27 at 1). */
-  P.hops = E.shape == WV_GROUP || (E.qs_host[0].n < 32768u && !E.qs_host[0].piece) ? 8u : 1u;
+  wv_schedule(P, E.shape, E.qs_host[0].n, E.qs_host[0].piece != nullptr);
   const bool grp = E.shape == WV_GROUP || E.shape == WV_POOL;
   P.filled = grp || (E.nq == 1u && E.qs_host[0].n > (1u << 18)) ? 1u : 0u;
   if (grp && cudaMemsetAsync(E.grp, 0, WV_GRP_WORDS * 4, st) != cudaSuccess) return -5;
@@ -1009,12 +1028,7 @@ int wv_engine_enqueue(WvEngine &E, unsigned single_src, unsigned long long timeo
     wave_fill<<<1184, 256, 0, st>>>(E.qs, single_src,
                                     E.flt ? ADDS_INF_F32_BITSV : ADDS_INF_I32_BITS);
   if (k0 && cudaEventRecordWithFlags(k0, st, fl) != cudaSuccess) return -5;
-  cudaError_t e = cudaErrorInvalidValue;
-#define X(s, b, ns, m, g, pl, lo) \
-  if (E.shape == s) e = E.flt ? launch<true, b, ns, m, g, pl>(P, st) : launch<false, b, ns, m, g, pl>(P, st);
-  WV_SHAPES(X)
-#undef X
-  if (e != cudaSuccess) return -5;
+  if (wv_launch(P, E.flt, E.shape, st) != cudaSuccess) return -5;
   if (k1 && cudaEventRecordWithFlags(k1, st, fl) != cudaSuccess) return -5;
   if (cudaMemcpyAsync(E.st_host, E.st, sizeof(WvStat), cudaMemcpyDeviceToHost, st) != cudaSuccess)
     return -5;

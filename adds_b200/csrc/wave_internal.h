@@ -14,6 +14,7 @@
 /* error word of a launch (first one wins) */
 #define WV_ERR_OVERFLOW 1u /* a list outgrew its area: solve on another engine */
 #define WV_ERR_TIMEOUT 2u
+#define WV_ERR_INPUT 3u    /* nothing to solve: the caller's arrays are invalid   */
 
 #define WV_PIECE 512u     /* edges of a long row one entry stands for          */
 #define WV_MAX_GROUP 160u /* CTAs of one group (a multiple of 32)              */
@@ -91,6 +92,14 @@ struct WvEngine {
 #define WV_GROUP 2
 #define WV_POOL 3
 #define WV_LAST WV_POOL
+
+/* the kernels themselves (noalloc.cu brings its own memory): residency of a
+ * variant (needed before its first launch), the schedule's parameters for P's
+ * group size, a launch, and a CTA's frontier entries in shared memory */
+cudaError_t wv_prepare(bool flt, int shape, int *ctas_per_sm);
+void wv_schedule(WvParams &P, int shape, unsigned n, bool pieces);
+cudaError_t wv_launch(const WvParams &P, bool flt, int shape, cudaStream_t st);
+unsigned wv_near(int shape);
 
 int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize,
                     const std::vector<WvQuery> &qv, cudaStream_t st);
