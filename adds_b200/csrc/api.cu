@@ -416,6 +416,7 @@ struct adds_graph {
   bool wave_off = false; /* their lists overflowed on this graph           */
   unsigned *wfirst = nullptr; /* pieces of long rows (WvQuery)              */
   uint4 *wpiece = nullptr;
+  unsigned wpieces = 0;
   unsigned trace_cap = 0; /* phase trace records requested (0 = off)       */
   PhParams last_pp;
   int last_engine = 0; /* engine of the solves in flight                   */
@@ -1366,6 +1367,7 @@ static int graph_pieces(adds_graph *g) {
     k_pieces<<<592, 256, 0, g->stream>>>(g->row, g->n, cnt, g->wfirst, g->wpiece);
     e = cudaGetLastError();
   }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&g->wpieces, cnt, 4, cudaMemcpyDeviceToHost, g->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
   if (e != cudaSuccess) {
     if (g->wpiece) cudaFree(g->wpiece);
@@ -1389,16 +1391,28 @@ static int graph_wave_engine(adds_graph *g, const Knobs &k, int shift, float sca
   memset(&q, 0, sizeof q);
   q.row = g->row;
   q.edges = g->edges;
+  /* Light and heavy edges apart: a hub that is improved again within a bucket
+   * relaxes its light edges only.  For graphs with long rows that are large
+   * enough for edges rather than hops to count (R-MAT 20 0.85 ms against 1.2
+   * with whole rows, R-MAT 18 0.62 both, R-MAT 16 0.49 against 0.41: the
+   * heavy hops are extra); ER 10^6 x 8 1.0 against 0.56. */
+  if (k.wave == WV_POOL &&
+      (k.light_heavy == 1 || (k.light_heavy == 2 && g->max_deg > WV_PIECE && g->n > (1u << 18)))) {
+    const int rl = graph_layout(g, k, shift, scale, &q.edges, &q.split);
+    if (rl) return rl;
+  }
   q.first = g->wfirst;
   q.piece = g->wpiece;
+  q.np = g->wpieces;
   q.dist = g->dist;
   q.n = g->n;
   q.m = g->m;
   q.delta = wave_delta(g, shift, scale);
   WvEngine &E = g->weng;
   const unsigned gs = (unsigned)std::max(0, k.group_ctas);
-  if (E.nq == 1 && E.shape == k.wave && E.req_gsize == gs) {
-    if (E.qs_host[0].delta == q.delta) return ADDS_OK;
+  if (E.nq == 1 && E.shape == k.wave && E.req_gsize == gs && (E.has_set || !q.split)) {
+    const WvQuery &h = E.qs_host[0];
+    if (h.delta == q.delta && h.edges == q.edges && h.split == q.split) return ADDS_OK;
     E.qs_host[0] = q;
     return wv_engine_upload(E, g->stream) ? ADDS_ERR_CUDA : ADDS_OK;
   }
@@ -1521,16 +1535,17 @@ static cudaStream_t pick_stream(const adds_graph *g, const adds_opts *o) {
  *   against 14.9 (1.8), 4096^2 18.3 against 310 (38); one CTA below 4,096
  *   vertices, where a group's exchanges cost what its width saves (16^2 0.107
  *   against 0.118, 64^2 0.295 against 0.25);
- *   longer rows: ER 4,001 x 8 0.16 against 0.57 (0.29), ER 10^6 x 8 0.6 against
- *   1.8 (0.95), R-MAT 16 0.38 against 0.87 (0.49), R-MAT 20 1.3 against 1.8
- *   (1.15).  The wave kernel relaxes whole rows (3 to 5 times each edge of an
- *   R-MAT graph), so from 2^25 edges on the phase engine's light/heavy split
- *   and pull phases win. */
+ *   longer rows: ER 4,001 x 8 0.16 against 0.57 (0.29), ER 10^6 x 8 0.56 against
+ *   1.7 (0.95), R-MAT 16 0.38 against 0.84 (0.49), R-MAT 20 0.85 against 1.8
+ *   (1.15), R-MAT 22 1.7 against 1.9, float 2.0 against 2.4; R-MAT 23 2.55 against
+ *   2.25: from there the phase engine's pull phases win, which relax half the
+ *   edges. */
 static int auto_wave(const adds_graph *g, const adds_opts *o) {
   if (g->wave_off || g->trace_cap || !schedule_auto(o)) return -1;
   if (g->tuned) return g->tuned_opts.wave > 0 ? g->tuned_opts.wave - 1 : -1;
   if (g->avg_deg < 6.0 && g->m < (1ull << 31)) return g->n < 4096u ? WV_WIDE : WV_GROUP;
-  return g->m < (1ull << 25) ? WV_POOL : -1;
+  if (g->n < 32768u && g->max_deg <= WV_PIECE) return WV_GROUP; /* ER 4,001 x 8: 0.15, pooled 0.18 */
+  return g->m < 100000000ull ? WV_POOL : -1;
 }
 
 /* Enqueues one solve; no host synchronisation.  Each solve records four
@@ -1894,6 +1909,7 @@ static int batch_wave_engine(adds_batch *b) {
     q.edges = g->edges;
     q.first = g->wfirst;
     q.piece = g->wpiece;
+    q.np = g->wpieces;
     q.dist = b->dist_all + b->dist_off[i];
     q.n = g->n;
     q.m = g->m;

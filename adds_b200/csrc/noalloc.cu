@@ -175,7 +175,8 @@ __global__ void na_setup(unsigned char *B, PhQuery desc, int is_float, unsigned 
   q.n = desc.n;
   q.src = desc.src;
   q.delta = is_float ? (float)((double)(1ull << shift) / (double)desc.scale) : (float)(1ull << shift);
-  q.pad = 0u;
+  q.np = kMaxPieces;
+  q.split = nullptr; /* every row is relaxed whole */
   q.m = desc.m;
   *(WvQuery *)(B + kOffWq) = q;
   if (bad != 0u) {

@@ -42,6 +42,16 @@
  * one batch 97.7 -> 7.2 ms; 60 sources on a 257 x 255 road 4.7 -> 1.6 ms; R-MAT 16
  * 0.87 -> 0.37 ms; ER 4,001 x 8 0.57 -> 0.15 ms.
  *
+ * Graphs with long rows (POOL): rows are cut into pieces that exchanges deal
+ * out, a CTA pools the edges of its entries over its threads, and on large
+ * graphs light and heavy edges are relaxed apart: heavy edges (which cannot
+ * land in the bucket that is being settled) once per settled vertex, when the
+ * frontier has run low.  R-MAT 20 relaxes 1.0 to 1.3 times its edges so, 3.5 to
+ * 4 times with whole rows; 0.85 ms against 1.2, and 1.8 on the phase engine.
+ * A full hop is bound by scattered requests (gathers 1,900, atomics 2,000, row
+ * searches and edge loads 2,500, pushes 1,400 cycles for 4,096 edges of an SM),
+ * a small one by its round trips.
+ *
  * The lists cannot grow: an overflow ends the launch with WV_ERR_OVERFLOW and
  * the host solves on another engine.
  */
@@ -66,7 +76,7 @@ __device__ __forceinline__ unsigned long long gtimer() {
 
 /* what the CTAs of a group tell each other at an exchange */
 struct __align__(16) Note {
-  unsigned near_cnt, far_cnt, far_min, stop;
+  unsigned near_cnt, far_cnt, far_min, stop; /* stop: errors, WV_SETTLED     */
 };
 
 /* a hop's pushes: entries of the next frontier, far entries added, error.
@@ -74,7 +84,9 @@ struct __align__(16) Note {
  * clears for the next, so that a hop needs one barrier. */
 struct __align__(16) Ctr {
   unsigned near_cnt, far_new, stop;
-  unsigned cut; /* a long row became pieces */
+  unsigned cut;     /* a long row became pieces                               */
+  unsigned set_new; /* settled entries added                                  */
+  unsigned pad[3];
 };
 
 template <int BLOCK, int NS, bool POOL>
@@ -82,6 +94,7 @@ struct WSmem {
   uint2 nb[2][NS];  /* frontier entries (v, d): this hop's, the next          */
   Ctr ctr[3];
   Note tot;         /* the group's totals                                     */
+  unsigned far_max; /* the longest far list of a CTA                          */
   unsigned kept;    /* far entries a split has kept                           */
   unsigned fmin;    /* the smallest distance among them                       */
   unsigned q, r0;
@@ -95,7 +108,8 @@ struct WSmem {
 struct Lists {
   uint2 *over;      /* frontier entries past the shared ones: two areas       */
   uint2 *far;
-  unsigned ncap, fcap;
+  uint2 *set;       /* settled entries (light/heavy split)                    */
+  unsigned ncap, fcap, scap;
 };
 
 template <bool FLT>
@@ -149,12 +163,14 @@ struct Wave {
     const uint2 *edges;
     const unsigned *first; /* long rows: a row's first piece, the pieces       */
     const uint4 *piece;
+    const unsigned *split; /* light edges at the start of each row, or null    */
     unsigned *dist;
-    unsigned n;
+    unsigned n, np;
     unsigned T;    /* near threshold (distance word)                          */
     unsigned cur;  /* frontier buffer being read                              */
     unsigned ci;   /* counter of that frontier                                */
     unsigned F;    /* far entries of this CTA                                 */
+    unsigned H;    /* settled entries of this CTA                             */
     unsigned npush, nstale;
     unsigned long long nedge;
   };
@@ -297,24 +313,106 @@ struct Wave {
     }
   }
 
+  /* A pooled hop's entry.  With the light/heavy split (rows sorted by weight)
+   * an id below n is a vertex whose light edges are wanted, then come the light
+   * pieces of long rows, their heavy pieces, and vertices whose heavy edges
+   * are.  set: the vertex joins the settled list, for its heavy edges.  Rows
+   * longer than a piece are cut here, deg is 0 for them. */
+  static __device__ __forceinline__ void load_pool(Smem &S, State &w, uint2 x, bool in,
+                                                   unsigned &r0, unsigned &deg, bool &set) {
+    r0 = deg = 0u;
+    set = false;
+    if (!in) return;
+    unsigned v = x.x, j0 = 0, len = 0;
+    const bool whole = v < w.n || v >= w.n + 2u * w.np;
+    bool heavy = v >= w.n + w.np;
+    if (whole) {
+      if (heavy) v -= w.n + 2u * w.np;
+      r0 = __ldg(w.row + v);
+      len = __ldg(w.row + v + 1) - r0;
+      deg = len;
+      if (w.split) {
+        const unsigned nl = __ldg(w.split + v);
+        set = !heavy && nl < len;
+        j0 = heavy ? nl / WV_PIECE : 0u;
+        deg = heavy ? len - nl : nl;
+        len = heavy ? len : nl; /* pieces from j0 on reach as far as this */
+        if (heavy) r0 += nl;
+      }
+    } else {
+      const uint4 c = __ldg(w.piece + (v - w.n - (heavy ? w.np : 0u)));
+      v = c.x;
+      r0 = c.y;
+      deg = c.z;
+      if (w.split) {
+        const unsigned off = c.y - __ldg(w.row + v), nl = __ldg(w.split + v);
+        if (heavy && nl > off) {
+          r0 += nl - off;
+          deg -= nl - off;
+        } else if (!heavy) {
+          deg = min(deg, nl - off);
+        }
+      }
+    }
+    if (__ldcg(w.dist + v) != x.y) {
+      ++w.nstale;
+      deg = 0u;
+      set = false;
+    } else if (whole && deg > WV_PIECE) {
+      Ctr &C = S.ctr[next3(w.ci)];
+      const unsigned j1 = (len + WV_PIECE - 1u) / WV_PIECE, k = j1 - j0;
+      const unsigned c0 = w.n + (heavy ? w.np : 0u) + __ldg(w.first + v) + j0;
+      const unsigned at = atomicAdd(&C.near_cnt, k);
+      if (at + k > NS + w.L.ncap) C.stop = WV_ERR_OVERFLOW;
+      C.cut = 1u;
+      for (unsigned j = 0; j < k; ++j) put(S, w, w.cur ^ 1u, at + j, make_uint2(c0 + j, x.y));
+      deg = 0u;
+    }
+  }
+
+  /* Ends a bucket: the settled entries that are still current become frontier
+   * entries for their heavy edges.  Uniform over the CTA. */
+  static __device__ void unsettle(Smem &S, State &w) {
+    const unsigned tid = threadIdx.x, lane = tid & 31u, lt = (1u << lane) - 1u;
+    Ctr &C = S.ctr[w.ci];
+    for (unsigned i0 = 0; i0 < w.H; i0 += BLOCK) {
+      const bool have = i0 + tid < w.H;
+      const uint2 x = have ? __ldcg(w.L.set + i0 + tid) : make_uint2(0u, 0u);
+      const bool in = have && __ldcg(w.dist + x.x) == x.y;
+      const unsigned b = __ballot_sync(0xFFFFFFFFu, in);
+      if (b == 0u) continue;
+      unsigned at = 0;
+      if (lane == 0) at = atomicAdd(&C.near_cnt, (unsigned)__popc(b));
+      at = __shfl_sync(0xFFFFFFFFu, at, 0);
+      if (at + __popc(b) > NS + w.L.ncap) C.stop = WV_ERR_OVERFLOW;
+      if (in) put(S, w, w.cur, at + __popc(b & lt), make_uint2(x.x + w.n + 2u * w.np, x.y));
+    }
+    w.H = 0u;
+    __syncthreads();
+  }
+
   /* A hop whose edges are pooled over the CTA: a block scan of the row
    * lengths, then every warp walks 32 x U neighbouring edges at a time. */
   static __device__ __forceinline__ void hop_pool(Smem &S, State &w, unsigned cnt) {
     constexpr int U = 4;
-    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    if (tid == 0) S.ctr[next3(next3(w.ci))] = Ctr{0u, 0u, 0u, 0u};
+    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, lt = (1u << lane) - 1u;
+    if (tid == 0) S.ctr[next3(next3(w.ci))] = Ctr{};
     for (unsigned i0 = 0; i0 < cnt; i0 += BLOCK) {
       const bool in = i0 + tid < cnt;
       const uint2 x = in ? entry(S, w, i0 + tid) : make_uint2(0u, 0u);
       unsigned r0, deg;
-      bool live;
-      load(w, x, in, r0, deg, live);
-      if (in && !live) ++w.nstale;
-      if (deg > WV_PIECE && x.x < w.n) {
-        if (live) cut(S, w, x, deg);
-        deg = 0u;
+      bool set;
+      load_pool(S, w, x, in, r0, deg, set);
+      const unsigned sb = __ballot_sync(0xFFFFFFFFu, set);
+      if (sb) {
+        unsigned at = 0;
+        if (lane == 0) at = atomicAdd(&S.ctr[next3(w.ci)].set_new, (unsigned)__popc(sb));
+        at = __shfl_sync(0xFFFFFFFFu, at, 0) + w.H + __popc(sb & lt);
+        if (set) {
+          if (at < w.L.scap) __stcg(w.L.set + at, x);
+          else S.ctr[next3(w.ci)].stop = WV_ERR_OVERFLOW;
+        }
       }
-      if (!live) deg = 0u;
       unsigned off = deg;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -342,7 +440,9 @@ struct Wave {
        * so its row is at most a few items on */
       const unsigned run = ((E + BLOCK / 32u - 1u) / (BLOCK / 32u) + 31u) & ~31u;
       const unsigned re = min(E, (warp + 1u) * run);
-      unsigned lo = 0; /* item of the lane's last edge: its edges only move forward */
+      /* item of the lane's last edge (its edges only move forward), where the
+       * item's edges end, and its row and distance */
+      unsigned lo = 0, fin = 0, shift_r = 0, dcur = 0;
       for (unsigned e0 = warp * run; e0 < re; e0 += 32u * U) {
         uint2 e[U];
         unsigned dd[U], msk = 0;
@@ -350,22 +450,26 @@ struct Wave {
         for (int u = 0; u < U; ++u) {
           const unsigned j = e0 + u * 32u + lane;
           e[u] = make_uint2(0u, 0u);
-          dd[u] = 0u;
           if (j < re) {
-            unsigned step = 1u;
-            while (lo + step < k && S.it_off[lo + step] <= j) {
-              lo += step;
-              step <<= 1;
+            if (j >= fin) {
+              unsigned step = 1u;
+              while (lo + step < k && S.it_off[lo + step] <= j) {
+                lo += step;
+                step <<= 1;
+              }
+              unsigned hi = min(lo + step, k) - 1u;
+              while (lo < hi) {
+                const unsigned mid = (lo + hi + 1u) >> 1;
+                if (S.it_off[mid] <= j) lo = mid; else hi = mid - 1u;
+              }
+              fin = lo + 1u < k ? S.it_off[lo + 1u] : E;
+              shift_r = S.it_r0[lo] - S.it_off[lo];
+              dcur = S.it_d[lo];
             }
-            unsigned hi = min(lo + step, k) - 1u;
-            while (lo < hi) {
-              const unsigned mid = (lo + hi + 1u) >> 1;
-              if (S.it_off[mid] <= j) lo = mid; else hi = mid - 1u;
-            }
-            e[u] = __ldg(w.edges + S.it_r0[lo] + (j - S.it_off[lo]));
-            dd[u] = S.it_d[lo];
+            e[u] = __ldg(w.edges + (shift_r + j));
             msk |= 1u << u;
           }
+          dd[u] = dcur;
         }
         relax<U>(S, w, e, dd, msk);
       }
@@ -377,7 +481,7 @@ struct Wave {
    * frontier and the far list.  The caller's barrier ends it. */
   static __device__ __forceinline__ void hop(Smem &S, State &w, unsigned cnt) {
     const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    if (tid == 0) S.ctr[next3(next3(w.ci))] = Ctr{0u, 0u, 0u, 0u};
+    if (tid == 0) S.ctr[next3(next3(w.ci))] = Ctr{};
     /* few entries: eight a warp, four lanes each, rows of up to eight edges in
      * one round, so that every warp of the CTA has part of the hop */
     const bool few = cnt <= BLOCK / 4u;
@@ -509,8 +613,8 @@ struct Wave {
     const unsigned tid = threadIdx.x, lane = tid & 31u, rank = blockIdx.x, G = P.gsize;
     const unsigned par = round & 1u, xcap = NS + w.L.ncap;
     /* areas are the same size for every CTA of a group */
-    const size_t stride = 2ull * w.L.ncap + w.L.fcap + 2ull * xcap;
-    uint2 *const mine = w.L.far + w.L.fcap + (size_t)par * xcap;
+    const size_t stride = 2ull * w.L.ncap + w.L.fcap + w.L.scap + 2ull * xcap;
+    uint2 *const mine = w.L.set + w.L.scap + (size_t)par * xcap;
     for (unsigned i = tid; i < min(cnt, xcap); i += BLOCK) __stcg(mine + i, entry(S, w, i));
     __syncthreads();
     /* The CTA's note carries the round: it is the arrival too.  One warp reads
@@ -520,17 +624,17 @@ struct Wave {
     ulonglong2 *const notes =
         reinterpret_cast<ulonglong2 *>(P.grp) + (size_t)par * WV_MAX_GROUP;
     ++round;
-    const unsigned tag = round << 2; /* low bits: the error */
+    const unsigned tag = round << 3; /* low bits: the error, WV_SETTLED */
     if (tid < 32u) {
       if (lane == 0) {
         __threadfence(); /* what the CTA published, before its note */
-        st_note(notes + rank, min(cnt, xcap), w.F, fmin, tag | stop);
+        st_note(notes + rank, min(cnt, xcap), w.F, fmin, tag | stop | (w.H ? WV_SETTLED : 0u));
       }
       constexpr unsigned J = WV_MAX_GROUP / 32u;
-      unsigned c[J], far = 0, fm = 0xFFFFFFFFu, st = 0, it = 0;
+      unsigned c[J], far = 0, fx = 0, fm = 0xFFFFFFFFu, st = 0, it = 0;
       bool late = false;
       for (;;) {
-        far = st = 0u;
+        far = fx = st = 0u;
         fm = 0xFFFFFFFFu;
         bool here = true;
 #pragma unroll
@@ -538,11 +642,12 @@ struct Wave {
           const unsigned r = j * 32u + lane;
           uint4 x = make_uint4(0u, 0u, 0xFFFFFFFFu, tag);
           if (r < G) x = ld_note(notes + r);
-          here = here && (x.w & ~3u) == tag;
+          here = here && (x.w & ~7u) == tag;
           c[j] = x.x;
           far += x.y;
+          fx = max(fx, x.y);
           fm = min(fm, x.z);
-          st = max(st, x.w & 3u);
+          st |= x.w & 7u; /* two errors at once count as the worse */
         }
         if (__all_sync(0xFFFFFFFFu, here)) break;
         late = (++it & 255u) == 0u && gtimer() > deadline;
@@ -566,8 +671,9 @@ struct Wave {
         if (j * 32u + lane < G) S.pre[j * 32u + lane] = c[j];
       }
       far = __reduce_add_sync(0xFFFFFFFFu, far);
+      fx = __reduce_max_sync(0xFFFFFFFFu, fx);
       fm = __reduce_min_sync(0xFFFFFFFFu, fm);
-      st = __reduce_max_sync(0xFFFFFFFFu, st);
+      st = __reduce_or_sync(0xFFFFFFFFu, st);
       /* first CTA whose entries reach into this CTA's share */
       const unsigned shr = ((tot + G - 1u) / G + 7u) & ~7u, lo = min(rank * shr, tot);
       unsigned first = 0;
@@ -576,6 +682,7 @@ struct Wave {
         first += __popc(__ballot_sync(0xFFFFFFFFu, j * 32u + lane < G && c[j] <= lo));
       if (lane == 0) {
         S.tot = Note{tot, far, fm, st};
+        S.far_max = fx;
         S.r0 = min(first, G - 1u);
         S.q = late ? 1u : 0u;
         if (late) atomicCAS(&P.st->err, 0u, WV_ERR_TIMEOUT);
@@ -593,7 +700,7 @@ struct Wave {
       r = 0u;
     }
     const uint2 *const base = reinterpret_cast<const uint2 *>(P.ws) + 2ull * w.L.ncap + w.L.fcap +
-                              (size_t)par * xcap;
+                              w.L.scap + (size_t)par * xcap;
     for (unsigned j = tid; j < hi - lo; j += BLOCK) {
       const unsigned i = lo + j * step; /* below tot = pre[G - 1] */
       if (POOL) {
@@ -608,8 +715,8 @@ struct Wave {
       put(S, w, w.cur, j, __ldcg(base + r * stride + (i - (r ? S.pre[r - 1] : 0u))));
     }
     if (tid == 0) {
-      S.ctr[w.ci] = Ctr{hi - lo, 0u, 0u, 0u};
-      S.ctr[next3(w.ci)] = Ctr{0u, 0u, 0u, 0u};
+      S.ctr[w.ci] = Ctr{hi - lo};
+      S.ctr[next3(w.ci)] = Ctr{};
       if (hi - lo > NS + w.L.ncap) S.ctr[w.ci].stop = WV_ERR_OVERFLOW;
     }
     __syncthreads();
@@ -625,8 +732,10 @@ struct Wave {
     State w;
     w.L.over = reinterpret_cast<uint2 *>(P.ws) + A.off;
     w.L.far = w.L.over + 2ull * A.ncap;
+    w.L.set = w.L.far + A.fcap;
     w.L.ncap = A.ncap;
     w.L.fcap = A.fcap;
+    w.L.scap = A.scap;
     w.npush = w.nstale = 0u;
     w.nedge = 0ull;
     unsigned err0 = *reinterpret_cast<volatile unsigned *>(&P.st->err), round = 0;
@@ -635,8 +744,8 @@ struct Wave {
       if (tid == 0) {
         const unsigned i = GRP ? turn : (turn == 0 ? blockIdx.x : atomicAdd(&P.st->next, 1u) + P.groups);
         S.q = i < P.nq ? P.order[i] : 0xFFFFFFFFu;
-        S.ctr[0] = Ctr{GRP && blockIdx.x != 0u ? 0u : 1u, 0u, err0, 0u};
-        S.ctr[1] = S.ctr[2] = Ctr{0u, 0u, 0u, 0u};
+        S.ctr[0] = Ctr{GRP && blockIdx.x != 0u ? 0u : 1u, 0u, err0};
+        S.ctr[1] = S.ctr[2] = Ctr{};
       }
       __syncthreads();
       const unsigned q = S.q;
@@ -646,6 +755,8 @@ struct Wave {
       w.edges = Q.edges;
       w.first = Q.first;
       w.piece = Q.piece;
+      w.split = Q.split;
+      w.np = Q.np;
       w.dist = Q.dist;
       w.n = Q.n;
       const unsigned src = (P.single_src != 0xFFFFFFFFu && q == 0u) ? P.single_src : Q.src;
@@ -665,7 +776,7 @@ struct Wave {
       __syncthreads();
       float delta = Q.delta;
       w.T = raise_word<FLT>(0u, delta);
-      w.cur = w.ci = w.F = 0u;
+      w.cur = w.ci = w.F = w.H = 0u;
       unsigned fmin = 0xFFFFFFFFu, hops = 0, split_at = 0, stop = 0;
       if (!GRP) {
         for (;;) {
@@ -705,15 +816,25 @@ struct Wave {
           w.ci = next3(w.ci);
         }
       } else {
+        /* A split leaves what it admits with the CTA that held it.  Where one
+         * CTA holds much more than the others (steps narrower than most
+         * weights: nothing of the first hops is dealt out) its entries are
+         * dealt out before they are relaxed (ER 300,000 x 16 with weights 1 to
+         * 10 overflowed the first CTA's list). */
+        bool deal = false;
         for (;;) {
           /* up to P.hops hops on this CTA's own entries */
+          const unsigned hmax = deal ? 0u : P.hops;
+          const bool dealt = deal;
+          deal = false;
           unsigned cnt = 0;
           for (unsigned h = 0;; ++h) {
             const Ctr c = S.ctr[w.ci];
             w.F += c.far_new;
+            w.H += c.set_new;
             cnt = c.near_cnt;
             stop = c.stop;
-            if (h == P.hops || cnt == 0u || stop != 0u || (h != 0u && (cnt > BLOCK / 2u || c.cut != 0u)))
+            if (h == hmax || cnt == 0u || stop != 0u || (h != 0u && (cnt > BLOCK / 2u || c.cut != 0u)))
               break;
             s_items += cnt;
             if (POOL) hop_pool(S, w, cnt); else hop(S, w, cnt);
@@ -727,17 +848,22 @@ struct Wave {
             break;
           }
           const Note t = S.tot;
-          stop = t.stop;
-          if (stop != 0u || (t.near_cnt == 0u && t.far_cnt == 0u)) break;
-          if (t.near_cnt <= P.low && t.far_cnt != 0u) {
-            if (round - split_at <= 1u) delta *= 1.5f;
+          stop = t.stop & ~WV_SETTLED;
+          const bool settled = (t.stop & WV_SETTLED) != 0u;
+          if (stop != 0u || (t.near_cnt == 0u && t.far_cnt == 0u && !settled)) break;
+          const bool few = t.near_cnt <= P.low && !(dealt && t.near_cnt != 0u);
+          if (POOL && few && settled) {
+            unsettle(S, w);
+          } else if (few && t.far_cnt != 0u) {
+            deal = S.far_max > 256u && (unsigned long long)S.far_max * P.gsize * 2u > 3ull * t.far_cnt;
+            if (P.grow && round - split_at <= 1u) delta *= 1.5f;
             split_at = round;
             w.T = raise_word<FLT>(
                 t.near_cnt == 0u && t.far_min != 0xFFFFFFFFu && t.far_min > w.T ? t.far_min : w.T, delta);
             split(S, w);
             fmin = S.fmin;
             ++s_splits;
-          } else if (t.near_cnt > P.high) {
+          } else if (P.grow && t.near_cnt > P.high) {
             delta *= 0.75f;
           }
           __syncthreads();
@@ -824,7 +950,7 @@ static cudaError_t launch(const WvParams &P, cudaStream_t st) {
   X(WV_CTA, 256, 1024, 4, false, false, 32)    \
   X(WV_WIDE, 1024, 4096, 1, false, false, 64)  \
   X(WV_GROUP, 512, 2048, 1, true, false, 16)   \
-  X(WV_POOL, 512, 2048, 1, true, true, 8)
+  X(WV_POOL, 1024, 2048, 1, true, true, 8)
 
 static unsigned wv_block(int shape) {
 #define X(s, b, ns, m, g, pl, lo) if (shape == s) return b;
@@ -890,6 +1016,7 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
   if (grp && E.nq != 1u) return -9;
   E.gsize = grp ? std::min(gsize ? gsize : (unsigned)sms, std::min((unsigned)sms, (unsigned)WV_MAX_GROUP)) : 1u;
   E.req_gsize = gsize;
+  E.has_set = shape == WV_POOL && qv[0].split != nullptr;
   E.groups = grp ? 1u : std::min((unsigned)(bps * sms), E.nq);
   E.ctas = E.groups * E.gsize;
   /* largest first: the last group to finish is not stuck with a big query */
@@ -921,9 +1048,12 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
         const unsigned long long n = maxn[g], cl = E.gsize;
         WvArea A;
         A.off = tot;
-        A.ncap = (unsigned)((dense ? n : n / 4u) / cl + std::min(n, 16384ull));
         A.fcap = (unsigned)((dense ? 4u * n : n / 2u) / cl + std::min(2ull * n, 65536ull));
+        /* a group's CTA may find its whole far list below a raised threshold */
+        A.ncap = grp ? A.fcap : (unsigned)((dense ? n : n / 4u) + std::min(n, 16384ull));
         tot += 2ull * A.ncap + A.fcap;
+        A.scap = shape == WV_POOL && qv[order[g]].split ? (unsigned)(2u * n / cl + std::min(n, 32768ull)) : 0u;
+        tot += A.scap;
         if (grp) tot += 2ull * (wv_near(shape) + A.ncap); /* published frontiers */
         area.push_back(A);
       }
@@ -967,6 +1097,11 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
 
 void wv_schedule(WvParams &P, int shape, unsigned n, bool pieces) {
   P.low = wv_low(shape) * P.gsize;
+  /* a pooled frontier widens its step only on small graphs, whose few hops are
+   * all latency: elsewhere a wide step relaxes rows again and again (ER 10^6 x 8
+   * 3.1 edges relaxed per edge and 0.90 ms with, 1.1 and 0.69 without; R-MAT 16
+   * 0.38 ms with, 0.42 without) */
+  P.grow = shape != WV_POOL || n < (1u << 17) ? 1u : 0u;
   P.high = wv_block(shape) * P.gsize * 4u;
   /* Hops on a CTA's own entries between two exchanges.  Roads: 8 (a 4096^2
    * grid 18.3 ms, against 19.3 at 4 and 33 at 1, where the exchanges cost more

@@ -16,13 +16,16 @@
 #define WV_ERR_TIMEOUT 2u
 #define WV_ERR_INPUT 3u    /* nothing to solve: the caller's arrays are invalid   */
 
+#define WV_SETTLED 4u     /* in a note: the CTA holds settled entries           */
 #define WV_PIECE 512u     /* edges of a long row one entry stands for          */
 #define WV_MAX_GROUP 160u /* CTAs of one group (a multiple of 32)              */
 #define WV_GRP_WORDS (2u * 4u * WV_MAX_GROUP) /* two sets of 16-byte notes     */
 
 struct WvQuery {
   const unsigned *row;
-  const uint2 *edges; /* rows in CSR order: nothing is sorted by weight        */
+  const uint2 *edges; /* rows in CSR order, or sorted by weight where split is  */
+  const unsigned *split; /* WV_POOL: light edges (w < delta) at the start of each
+                            row; null: every row is relaxed whole             */
   /* rows of more than WV_PIECE edges: their first piece by vertex, and the
    * pieces {vertex, first edge, edges, 0}; null where no row is that long */
   const unsigned *first;
@@ -31,7 +34,7 @@ struct WvQuery {
   unsigned n;
   unsigned src;
   float delta;        /* first step of the near threshold, in distance units   */
-  unsigned pad;
+  unsigned np;        /* pieces                                               */
   unsigned long long m;
 };
 
@@ -39,6 +42,7 @@ struct WvQuery {
 struct WvArea {
   unsigned long long off; /* two frontier overflow areas, then the far list    */
   unsigned ncap, fcap;    /* entries of one frontier overflow area / far list  */
+  unsigned scap, pad;     /* entries of the settled list                       */
 };
 
 struct WvStat {
@@ -57,6 +61,7 @@ struct WvParams {
   void *ws;
   WvStat *st;
   unsigned *grp;          /* a group's notes, two sets; cleared before a launch */
+  unsigned grow;          /* the threshold's step may widen                    */
   unsigned hops;          /* hops between two exchanges of a group             */
   unsigned single_src;    /* overrides query 0's source when != ~0             */
   unsigned filled;        /* the distances hold INF and the source already     */
@@ -82,6 +87,7 @@ struct WvEngine {
   WvStat *st = nullptr;
   WvStat *st_host = nullptr; /* pinned                                         */
   std::vector<WvQuery> qs_host;
+  bool has_set = false; /* room for settled lists                             */
   size_t bytes = 0;
 };
 

@@ -169,3 +169,39 @@ def test_batch_overflow_moves_to_an_engine():
     b.close()
     dg.close()
     dr.close()
+
+
+@pytest.mark.parametrize("wtype", [G.I32, G.F32])
+@pytest.mark.parametrize("shift", [-1, 0, 9, 31])
+def test_pooled_light_heavy(wtype, shift):
+    """Rows cut at any width: light and heavy parts empty, short, and longer
+    than a piece, on one CTA and on many."""
+    w = dict(wtype=wtype, w_lo=1, w_hi=1000)
+    r = G.rmat(13, 16, seed=6, **w)
+    rows = [PIECE - 1, PIECE + 1, 2 * PIECE + 3, 3000, 5, 0, 7000]
+    for ctas in (1, 5, 148):
+        kw = dict(wave=POOL, light_heavy=1, delta_shift=shift, group_ctas=ctas)
+        check(r, [G.max_degree_vertex(r), 11], **kw)
+        check(star(rows, wtype, seed=ctas), [0], **kw)
+    check(G.grid(60, 40, 0.02, 8, seed=8, **w), [7], wave=POOL, light_heavy=1, delta_shift=shift)
+
+
+def test_pooled_weights_of_few_values():
+    """Nearly every pending vertex falls below one raised threshold."""
+    g = G.erdos_renyi(60000, 16, w_lo=1, w_hi=3, seed=9)
+    for lh in (0, 1):
+        st = check(g, [1, 59999], wave=POOL, light_heavy=lh)
+        assert st["retries"] == 0
+
+
+def test_pooled_after_weight_update():
+    g = G.rmat(12, 16, seed=10)
+    dg = A.Graph.from_csr(g)
+    for seed in range(3):
+        w = np.random.default_rng(seed).integers(1, 900 if seed else 5, g.m).astype(np.uint32)
+        dg.set_weights(w)
+        n = G.CSR(g.n, g.row, g.dst, w, G.I32)
+        for lh in (0, 1):
+            d, _ = dg.sssp(9, A.default_opts(timeout_ms=10000, wave=POOL, light_heavy=lh))
+            assert np.array_equal(d, O.dijkstra(n, 9)[0])
+    dg.close()
