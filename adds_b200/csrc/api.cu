@@ -1384,23 +1384,30 @@ static float wave_delta(const adds_graph *g, int shift, float scale) {
   return (float)(g->wt == ADDS_F32 ? d / (double)scale : d);
 }
 
+/* The edges of a wave kernel's query, and where light ones end.  Light and
+ * heavy edges apart: a hub that is improved again within a bucket relaxes its
+ * light edges only.  For graphs with long rows that are large enough for edges
+ * rather than hops to count (R-MAT 20 0.85 ms against 1.2 with whole rows,
+ * R-MAT 18 0.62 both, R-MAT 16 0.49 against 0.41: the heavy hops are extra);
+ * ER 10^6 x 8 1.0 against 0.56. */
+static int wave_layout(adds_graph *g, const Knobs &k, int shift, float scale, const uint2 **edges,
+                       const unsigned **split) {
+  *edges = g->edges;
+  *split = nullptr;
+  if (k.wave != WV_POOL || k.light_heavy == 0 ||
+      (k.light_heavy == 2 && (g->max_deg <= WV_PIECE || g->n <= (1u << 18))))
+    return ADDS_OK;
+  return graph_layout(g, k, shift, scale, edges, split);
+}
+
 static int graph_wave_engine(adds_graph *g, const Knobs &k, int shift, float scale) {
   const int rp = graph_pieces(g);
   if (rp) return rp;
   WvQuery q;
   memset(&q, 0, sizeof q);
   q.row = g->row;
-  q.edges = g->edges;
-  /* Light and heavy edges apart: a hub that is improved again within a bucket
-   * relaxes its light edges only.  For graphs with long rows that are large
-   * enough for edges rather than hops to count (R-MAT 20 0.85 ms against 1.2
-   * with whole rows, R-MAT 18 0.62 both, R-MAT 16 0.49 against 0.41: the
-   * heavy hops are extra); ER 10^6 x 8 1.0 against 0.56. */
-  if (k.wave == WV_POOL &&
-      (k.light_heavy == 1 || (k.light_heavy == 2 && g->max_deg > WV_PIECE && g->n > (1u << 18)))) {
-    const int rl = graph_layout(g, k, shift, scale, &q.edges, &q.split);
-    if (rl) return rl;
-  }
+  const int rl = wave_layout(g, k, shift, scale, &q.edges, &q.split);
+  if (rl) return rl;
   q.first = g->wfirst;
   q.piece = g->wpiece;
   q.np = g->wpieces;
@@ -1414,6 +1421,7 @@ static int graph_wave_engine(adds_graph *g, const Knobs &k, int shift, float sca
     const WvQuery &h = E.qs_host[0];
     if (h.delta == q.delta && h.edges == q.edges && h.split == q.split) return ADDS_OK;
     E.qs_host[0] = q;
+    wv_query_schedule(E.qs_host[0], k.wave);
     return wv_engine_upload(E, g->stream) ? ADDS_ERR_CUDA : ADDS_OK;
   }
   const int rc = wv_engine_alloc(E, g->device, g->wt == ADDS_F32, k.wave, gs,
@@ -1841,6 +1849,7 @@ struct adds_batch {
   Engine eng;
   PhEngine peng; /* used when kn.engine is ADDS_ENGINE_PHASE */
   WvEngine weng; /* used when kn.wave names a variant */
+  unsigned wave_group = 0; /* CTAs per query of its group variants */
   PhParams pp;
   unsigned grow = 1;
   Knobs kn;
@@ -1906,7 +1915,8 @@ static int batch_wave_engine(adds_batch *b) {
     WvQuery q;
     memset(&q, 0, sizeof q);
     q.row = g->row;
-    q.edges = g->edges;
+    const int rl = wave_layout(g, b->kn, b->shifts[i], b->scales[i], &q.edges, &q.split);
+    if (rl) return rl;
     q.first = g->wfirst;
     q.piece = g->wpiece;
     q.np = g->wpieces;
@@ -1922,7 +1932,7 @@ static int batch_wave_engine(adds_batch *b) {
     b->exec = nullptr;
   }
   b->captured = false;
-  const int rc = wv_engine_alloc(b->weng, b->device, b->flt, b->kn.wave, 0u, qv, b->stream);
+  const int rc = wv_engine_alloc(b->weng, b->device, b->flt, b->kn.wave, b->wave_group, qv, b->stream);
   if (rc) snprintf(g_last_err, sizeof g_last_err, "wave kernel allocation failed (%d)", rc);
   return rc;
 }
@@ -2024,15 +2034,30 @@ extern "C" int adds_batch_create(adds_graph *const *graphs, const uint32_t *srcs
     int s_unused;
     float sc_unused;
     resolve(graphs[big], &lw, &b->kn, &s_unused, &sc_unused, false);
-    /* Sparse graphs with the schedule left to the library: one CTA per query
-     * on the wave kernels.  128 grids x 16 sources 7.3 ms against 98 on the
-     * asynchronous engine; 60 sources on a 257 x 255 road 1.6 against 4.7
-     * (1,024 threads a query while every query has an SM to itself: 2.4 ms
-     * with 256). */
-    bool sparse = schedule_auto(opts);
-    for (adds_graph *g : b->ugraph) sparse = sparse && g->avg_deg < 6.0 && g->m < (1ull << 31);
-    if (sparse) b->kn.wave = nq <= 148u ? WV_WIDE : WV_CTA;
-    if (b->kn.wave >= WV_GROUP && nq != 1u) b->kn.wave = WV_WIDE; /* groups solve one query */
+    /* With the schedule left to the library, the wave kernels (against the
+     * engine they stand in for).  Sparse graphs: four SMs or more a query while
+     * there are enough (15 queries on grids of side 61 to 130 0.47 ms, one SM
+     * each 0.53), an SM each up to 148 queries (60 on a 257 x 255 road 1.6 ms, two
+     * SMs each 2.0, the asynchronous engine 4.7), else four queries to an SM (128
+     * grids x 16 sources 7.3 ms against 98).  Others: groups of at least four SMs,
+     * which take the queries one after another (192 ER graphs and 64 sources on
+     * R-MAT 20 in groups of 1, 2, 4, 6, 9, 18: 38, 23.5, 21.9, 22.3, 22.8, 26.4 ms;
+     * phase engine 27.6). */
+    if (b->kn.wave < 0 && schedule_auto(opts)) {
+      bool sparse = true, fits = true;
+      for (adds_graph *g : b->ugraph) {
+        sparse = sparse && g->avg_deg < 6.0;
+        fits = fits && g->m < 100000000ull;
+      }
+      if (sparse) b->kn.wave = nq <= 37u ? WV_GROUP : (nq <= 148u ? WV_WIDE : WV_CTA);
+      else if (fits) b->kn.wave = WV_POOL;
+    }
+    if (b->kn.wave >= WV_GROUP) {
+      int sms = 0;
+      CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      b->wave_group = opts && opts->group_ctas > 0 ? (unsigned)opts->group_ctas
+                                                    : std::max(4u, (unsigned)sms / nq);
+    }
   }
   /* the batch sizes its groups itself unless the caller says otherwise */
   b->kn.group_ctas = (opts && opts->group_ctas > 0) ? opts->group_ctas : 0;
@@ -2111,9 +2136,20 @@ static int batch_relayout(adds_batch *b) {
   for (size_t i = 0; i < b->ugraph.size(); ++i)
     if (b->ugraph[i]->wversion != b->wversions[i]) changed = true;
   if (!changed) return ADDS_OK;
-  if (b->kn.wave >= 0) { /* the CSR itself, whose weights changed in place */
+  if (b->kn.wave >= 0) { /* the CSR itself, or the copy sorted by weight */
+    bool moved = false;
+    for (size_t i = 0; i < b->qgraph.size(); ++i) {
+      WvQuery &q = b->weng.qs_host[i];
+      const uint2 *edges;
+      const unsigned *split;
+      const int rc = wave_layout(b->qgraph[i], b->kn, b->shifts[i], b->scales[i], &edges, &split);
+      if (rc) return rc;
+      moved = moved || q.edges != edges || q.split != split;
+      q.edges = edges;
+      q.split = split;
+    }
     for (size_t i = 0; i < b->ugraph.size(); ++i) b->wversions[i] = b->ugraph[i]->wversion;
-    return ADDS_OK;
+    return moved && wv_engine_upload(b->weng, b->stream) ? ADDS_ERR_CUDA : ADDS_OK;
   }
   for (size_t i = 0; i < b->qgraph.size(); ++i) {
     const uint2 *edges;

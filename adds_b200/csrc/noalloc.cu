@@ -153,7 +153,7 @@ __global__ void na_clear(unsigned char *B) {
  * float keys are dist * 2^16 / mean weight (api.cu auto_scale).  Arrays
  * that failed validation set the error words instead, and the solvers exit
  * without touching them. */
-__global__ void na_setup(unsigned char *B, PhQuery desc, int is_float, unsigned ns) {
+__global__ void na_setup(unsigned char *B, PhQuery desc, WvQuery q, int is_float, unsigned ns) {
   const double wsum = *(const double *)(B + kOffSum);
   const unsigned bad = *(const unsigned *)(B + kOffSum + 8);
   PhGlobal *g = (PhGlobal *)(B + kOffG);
@@ -166,18 +166,7 @@ __global__ void na_setup(unsigned char *B, PhQuery desc, int is_float, unsigned 
   desc.shift = shift;
   desc.scale = (float)(65536.0 / aw);
   *(PhQuery *)(B + kOffQd) = desc;
-  WvQuery q;
-  q.row = desc.row;
-  q.edges = desc.edges;
-  q.first = (const unsigned *)(B + kOffFirst);
-  q.piece = (const uint4 *)(B + kOffPiece);
-  q.dist = desc.dist;
-  q.n = desc.n;
-  q.src = desc.src;
   q.delta = is_float ? (float)((double)(1ull << shift) / (double)desc.scale) : (float)(1ull << shift);
-  q.np = kMaxPieces;
-  q.split = nullptr; /* every row is relaxed whole */
-  q.m = desc.m;
   *(WvQuery *)(B + kOffWq) = q;
   if (bad != 0u) {
     g->err = PH_ERR_INPUT;
@@ -316,7 +305,20 @@ extern "C" int adds_sssp_noalloc(uint32_t n, uint64_t m, const uint32_t *row_sta
   desc.n = n;
   desc.src = src;
   desc.m = m;
-  na_setup<<<1, 1, 0, st>>>(B, desc, flt, ns);
+  WvQuery wq;
+  memset(&wq, 0, sizeof wq); /* split null: every row is relaxed whole */
+  wq.row = desc.row;
+  wq.edges = desc.edges;
+  wq.first = (const unsigned *)(B + kOffFirst);
+  wq.piece = (const uint4 *)(B + kOffPiece);
+  wq.np = kMaxPieces;
+  wq.dist = dist;
+  wq.n = n;
+  wq.src = src;
+  wq.m = m;
+  const int shape = m < 6ull * n ? WV_GROUP : WV_POOL;
+  wv_query_schedule(wq, shape);
+  na_setup<<<1, 1, 0, st>>>(B, desc, wq, flt, ns);
   NA_CK(cudaGetLastError());
 
   /* A wave kernel solves; where its lists do not suffice, the phase engine,
@@ -338,8 +340,7 @@ extern "C" int adds_sssp_noalloc(uint32_t n, uint64_t m, const uint32_t *row_sta
   W.single_src = 0xFFFFFFFFu;
   W.filled = 1u;
   W.timeout_ns = 20000ull * 1000000ull;
-  const int shape = m < 6ull * n ? WV_GROUP : WV_POOL;
-  wv_schedule(W, shape, n, true);
+  wv_schedule(W, shape);
   NA_CK(wv_launch(W, flt, shape, st));
   na_after<<<148, 256, 0, st>>>(B);
   NA_CK(cudaGetLastError());

@@ -610,7 +610,8 @@ struct Wave {
   static __device__ bool exchange(const WvParams &P, Smem &S, State &w, unsigned cnt,
                                   unsigned fmin, unsigned stop, unsigned &round,
                                   unsigned long long deadline) {
-    const unsigned tid = threadIdx.x, lane = tid & 31u, rank = blockIdx.x, G = P.gsize;
+    const unsigned tid = threadIdx.x, lane = tid & 31u, G = P.gsize;
+    const unsigned group = blockIdx.x / G, rank = blockIdx.x % G;
     const unsigned par = round & 1u, xcap = NS + w.L.ncap;
     /* areas are the same size for every CTA of a group */
     const size_t stride = 2ull * w.L.ncap + w.L.fcap + w.L.scap + 2ull * xcap;
@@ -622,7 +623,7 @@ struct Wave {
      * frontiers alternate between two areas, so a CTA that runs ahead does not
      * write over what a slower one still reads. */
     ulonglong2 *const notes =
-        reinterpret_cast<ulonglong2 *>(P.grp) + (size_t)par * WV_MAX_GROUP;
+        reinterpret_cast<ulonglong2 *>(P.grp) + ((size_t)group * 2u + par) * WV_MAX_GROUP;
     ++round;
     const unsigned tag = round << 3; /* low bits: the error, WV_SETTLED */
     if (tid < 32u) {
@@ -699,8 +700,7 @@ struct Wave {
       step = G;
       r = 0u;
     }
-    const uint2 *const base = reinterpret_cast<const uint2 *>(P.ws) + 2ull * w.L.ncap + w.L.fcap +
-                              w.L.scap + (size_t)par * xcap;
+    const uint2 *const base = mine - rank * stride; /* CTA 0 of the group      */
     for (unsigned j = tid; j < hi - lo; j += BLOCK) {
       const unsigned i = lo + j * step; /* below tot = pre[G - 1] */
       if (POOL) {
@@ -725,6 +725,8 @@ struct Wave {
 
   static __device__ void run(const WvParams &P, Smem &S) {
     const unsigned tid = threadIdx.x, lane = tid & 31u;
+    const unsigned rank = GRP ? blockIdx.x % P.gsize : 0u;
+    const unsigned group = GRP ? blockIdx.x / P.gsize : blockIdx.x;
     const WvArea A = P.area[blockIdx.x];
     const unsigned inf = FLT ? ADDS_INF_F32_BITSV : ADDS_INF_I32_BITS;
     const unsigned long long deadline = gtimer() + P.timeout_ns;
@@ -740,11 +742,13 @@ struct Wave {
     w.nedge = 0ull;
     unsigned err0 = *reinterpret_cast<volatile unsigned *>(&P.st->err), round = 0;
     for (unsigned turn = 0;; ++turn) {
-      /* a CTA's next query: its own first, then from the counter */
+      /* a CTA's next query: its own first, then from the counter; a group's:
+       * from its share of the order */
       if (tid == 0) {
-        const unsigned i = GRP ? turn : (turn == 0 ? blockIdx.x : atomicAdd(&P.st->next, 1u) + P.groups);
-        S.q = i < P.nq ? P.order[i] : 0xFFFFFFFFu;
-        S.ctr[0] = Ctr{GRP && blockIdx.x != 0u ? 0u : 1u, 0u, err0};
+        const unsigned i = GRP ? (P.qoff ? P.qoff[group] : 0u) + turn
+                               : (turn == 0 ? group : atomicAdd(&P.st->next, 1u) + P.groups);
+        S.q = i < (GRP && P.qoff ? P.qoff[group + 1u] : P.nq) ? P.order[i] : 0xFFFFFFFFu;
+        S.ctr[0] = Ctr{rank != 0u ? 0u : 1u, 0u, err0};
         S.ctr[1] = S.ctr[2] = Ctr{};
       }
       __syncthreads();
@@ -760,6 +764,10 @@ struct Wave {
       w.dist = Q.dist;
       w.n = Q.n;
       const unsigned src = (P.single_src != 0xFFFFFFFFu && q == 0u) ? P.single_src : Q.src;
+      if (GRP && !P.filled) { /* an exchange follows before the first hop */
+        for (unsigned i = rank * BLOCK + tid; i < Q.n; i += P.gsize * BLOCK)
+          __stcg(Q.dist + i, i == src ? 0u : inf);
+      }
       if (!GRP && !P.filled) {
         if ((reinterpret_cast<unsigned long long>(Q.dist) & 15ull) == 0ull) {
           const unsigned n4 = Q.n >> 2;
@@ -777,7 +785,7 @@ struct Wave {
       float delta = Q.delta;
       w.T = raise_word<FLT>(0u, delta);
       w.cur = w.ci = w.F = w.H = 0u;
-      unsigned fmin = 0xFFFFFFFFu, hops = 0, split_at = 0, stop = 0;
+      unsigned fmin = 0xFFFFFFFFu, hops = 0, split_at = GRP ? round : 0u, stop = 0;
       if (!GRP) {
         for (;;) {
           const Ctr c = S.ctr[w.ci];
@@ -821,10 +829,10 @@ struct Wave {
          * weights: nothing of the first hops is dealt out) its entries are
          * dealt out before they are relaxed (ER 300,000 x 16 with weights 1 to
          * 10 overflowed the first CTA's list). */
-        bool deal = false;
+        bool deal = !P.filled;
         for (;;) {
           /* up to P.hops hops on this CTA's own entries */
-          const unsigned hmax = deal ? 0u : P.hops;
+          const unsigned hmax = deal ? 0u : Q.hops;
           const bool dealt = deal;
           deal = false;
           unsigned cnt = 0;
@@ -856,18 +864,18 @@ struct Wave {
             unsettle(S, w);
           } else if (few && t.far_cnt != 0u) {
             deal = S.far_max > 256u && (unsigned long long)S.far_max * P.gsize * 2u > 3ull * t.far_cnt;
-            if (P.grow && round - split_at <= 1u) delta *= 1.5f;
+            if (Q.grow && round - split_at <= 1u) delta *= 1.5f;
             split_at = round;
             w.T = raise_word<FLT>(
                 t.near_cnt == 0u && t.far_min != 0xFFFFFFFFu && t.far_min > w.T ? t.far_min : w.T, delta);
             split(S, w);
             fmin = S.fmin;
             ++s_splits;
-          } else if (P.grow && t.near_cnt > P.high) {
+          } else if (Q.grow && t.near_cnt > P.high) {
             delta *= 0.75f;
           }
           __syncthreads();
-          if (gtimer() > deadline && tid == 0 && blockIdx.x == 0) S.ctr[w.ci].stop = WV_ERR_TIMEOUT;
+          if (gtimer() > deadline && tid == 0 && rank == 0u) S.ctr[w.ci].stop = WV_ERR_TIMEOUT;
           __syncthreads();
         }
       }
@@ -889,7 +897,7 @@ struct Wave {
       if (s_stale) atomicAdd(&P.st->stale, s_stale);
       if (tid == 0) {
         atomicAdd(&P.st->items, s_items);
-        if (!GRP || blockIdx.x == 0u) {
+        if (rank == 0u) {
           atomicAdd(&P.st->steps, GRP ? (unsigned long long)round : s_hops);
           atomicAdd(&P.st->splits, s_splits);
         }
@@ -1013,11 +1021,12 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
     return -9;
   }
   const bool grp = shape == WV_GROUP || shape == WV_POOL;
-  if (grp && E.nq != 1u) return -9;
+  for (WvQuery &q : E.qs_host) wv_query_schedule(q, shape);
   E.gsize = grp ? std::min(gsize ? gsize : (unsigned)sms, std::min((unsigned)sms, (unsigned)WV_MAX_GROUP)) : 1u;
   E.req_gsize = gsize;
-  E.has_set = shape == WV_POOL && qv[0].split != nullptr;
-  E.groups = grp ? 1u : std::min((unsigned)(bps * sms), E.nq);
+  E.has_set = false;
+  for (const WvQuery &q : qv) E.has_set = E.has_set || (shape == WV_POOL && q.split);
+  E.groups = grp ? std::min((unsigned)sms / E.gsize, E.nq) : std::min((unsigned)(bps * sms), E.nq);
   E.ctas = E.groups * E.gsize;
   /* largest first: the last group to finish is not stuck with a big query */
   std::vector<unsigned> order(E.nq);
@@ -1025,6 +1034,25 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
   std::stable_sort(order.begin(), order.end(), [&](unsigned a, unsigned b) {
     return qv[a].m + qv[a].n > qv[b].m + qv[b].n;
   });
+  /* Several groups: each its own share of the queries, the next largest one to
+   * the group with the least to do so far (edges, and the hops of any query
+   * as 500,000 edges a CTA). */
+  std::vector<unsigned> qoff;
+  if (grp && E.nq > 1u) {
+    std::vector<std::vector<unsigned>> share(E.groups);
+    std::vector<double> load(E.groups, 0.0);
+    for (unsigned i : order) {
+      const size_t g = std::min_element(load.begin(), load.end()) - load.begin();
+      share[g].push_back(i);
+      load[g] += (double)qv[i].m + 5e5 * E.gsize;
+    }
+    order.clear();
+    for (const auto &v : share) {
+      qoff.push_back((unsigned)order.size());
+      order.insert(order.end(), v.begin(), v.end());
+    }
+    qoff.push_back((unsigned)order.size());
+  }
   /* A CTA's lists hold the queries it may meet: its own first one and any
    * later one.  A road's wave front is a small part of its graph: frontier
    * n/4 (and the shared entries) and far list n/2 in all.  A graph with longer
@@ -1039,6 +1067,11 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
     mx = std::max(mx, qv[order[i]].n);
     maxn[i] = mx;
   }
+  if (!qoff.empty()) /* a group meets its own share only, the largest first */
+    for (unsigned g = 0; g < E.groups; ++g) {
+      maxn[g] = 0;
+      for (unsigned i = qoff[g]; i < qoff[g + 1]; ++i) maxn[g] = std::max(maxn[g], qv[order[i]].n);
+    }
   unsigned long long tot = 0;
   for (;;) {
     area.clear();
@@ -1048,18 +1081,21 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
         const unsigned long long n = maxn[g], cl = E.gsize;
         WvArea A;
         A.off = tot;
-        A.fcap = (unsigned)((dense ? 4u * n : n / 2u) / cl + std::min(2ull * n, 65536ull));
+        /* (side by side, half of that: the lists of a group of two CTAs on a
+         * graph of 10^6 vertices take 50 MB) */
+        A.fcap = (unsigned)((dense ? (E.groups > 1u ? 2u : 4u) * n : n / 2u) / cl +
+                            std::min(dense ? 2ull * n : n, dense ? 65536ull : 32768ull));
         /* a group's CTA may find its whole far list below a raised threshold */
-        A.ncap = grp ? A.fcap : (unsigned)((dense ? n : n / 4u) + std::min(n, 16384ull));
+        A.ncap = grp ? (E.groups > 1u ? A.fcap / 2u : A.fcap) : (unsigned)((dense ? n : n / 4u) + std::min(n, 16384ull));
         tot += 2ull * A.ncap + A.fcap;
-        A.scap = shape == WV_POOL && qv[order[g]].split ? (unsigned)(2u * n / cl + std::min(n, 32768ull)) : 0u;
+        A.scap = E.has_set ? (unsigned)((E.groups > 1u ? 1u : 2u) * n / cl + std::min(n, 32768ull)) : 0u;
         tot += A.scap;
         if (grp) tot += 2ull * (wv_near(shape) + A.ncap); /* published frontiers */
         area.push_back(A);
       }
     /* at most 8 GB of lists: fewer queries side by side, if need be */
     if (tot <= (1ull << 30)) break;
-    if (E.groups <= 8u) return -4;
+    if (grp || E.groups <= 8u) return -4;
     E.groups /= 2u;
   }
   E.ctas = E.groups * E.gsize;
@@ -1074,11 +1110,11 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
     E.bytes += _b;                                        \
   } while (0)
   WV_ALLOC(E.qs, (size_t)E.nq * sizeof(WvQuery));
-  WV_ALLOC(E.order, (size_t)E.nq * 4);
+  WV_ALLOC(E.order, (size_t)(E.nq + E.groups + 1u) * 4);
   WV_ALLOC(E.area, (size_t)E.ctas * sizeof(WvArea));
   WV_ALLOC(E.ws, (size_t)tot * 8);
   WV_ALLOC(E.st, sizeof(WvStat));
-  WV_ALLOC(E.grp, WV_GRP_WORDS * 4);
+  WV_ALLOC(E.grp, (size_t)E.groups * WV_GRP_WORDS * 4);
 #undef WV_ALLOC
   if (cudaMallocHost((void **)&E.st_host, sizeof(WvStat)) != cudaSuccess) {
     cudaGetLastError();
@@ -1086,7 +1122,9 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
     return -4;
   }
   memset(E.st_host, 0, sizeof(WvStat));
-  if (cudaMemcpyAsync(E.order, order.data(), (size_t)E.nq * 4, cudaMemcpyHostToDevice, st) !=
+  E.shares = !qoff.empty();
+  order.insert(order.end(), qoff.begin(), qoff.end());
+  if (cudaMemcpyAsync(E.order, order.data(), order.size() * 4, cudaMemcpyHostToDevice, st) !=
           cudaSuccess ||
       cudaMemcpyAsync(E.area, area.data(), area.size() * sizeof(WvArea), cudaMemcpyHostToDevice,
                       st) != cudaSuccess)
@@ -1095,21 +1133,24 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
   return rc ? rc : wv_engine_reset(E, st);
 }
 
-void wv_schedule(WvParams &P, int shape, unsigned n, bool pieces) {
+void wv_schedule(WvParams &P, int shape) {
   P.low = wv_low(shape) * P.gsize;
-  /* a pooled frontier widens its step only on small graphs, whose few hops are
-   * all latency: elsewhere a wide step relaxes rows again and again (ER 10^6 x 8
-   * 3.1 edges relaxed per edge and 0.90 ms with, 1.1 and 0.69 without; R-MAT 16
-   * 0.38 ms with, 0.42 without) */
-  P.grow = shape != WV_POOL || n < (1u << 17) ? 1u : 0u;
   P.high = wv_block(shape) * P.gsize * 4u;
+}
+
+void wv_query_schedule(WvQuery &q, int shape) {
   /* Hops on a CTA's own entries between two exchanges.  Roads: 8 (a 4096^2
    * grid 18.3 ms, against 19.3 at 4 and 33 at 1, where the exchanges cost more
    * than the hops).  Pooled: 1, since the neighbours of an entry are anywhere
    * and hops on stale distances relax too much (R-MAT 16 0.38 ms, 0.60 at 8),
    * but 8 on graphs so small that the few hops are all there is (20,000
    * vertices 0.20 ms, 0.27 at 1). */
-  P.hops = shape == WV_GROUP || (n < 32768u && !pieces) ? 8u : 1u;
+  q.hops = shape == WV_GROUP || (q.n < 32768u && !q.piece) ? 8u : 1u;
+  /* a pooled frontier widens its step only on small graphs, whose few hops are
+   * all latency: elsewhere a wide step relaxes rows again and again (ER 10^6 x 8
+   * 3.1 edges relaxed per edge and 0.90 ms with, 1.1 and 0.69 without; R-MAT 16
+   * 0.38 ms with, 0.42 without) */
+  q.grow = shape != WV_POOL || q.n < (1u << 17) ? 1u : 0u;
 }
 
 cudaError_t wv_prepare(bool flt, int shape, int *bps) {
@@ -1146,6 +1187,7 @@ int wv_engine_enqueue(WvEngine &E, unsigned single_src, unsigned long long timeo
   memset(&P, 0, sizeof P);
   P.qs = E.qs;
   P.order = E.order;
+  P.qoff = E.shares ? E.order + E.nq : nullptr;
   P.nq = E.nq;
   P.groups = E.groups;
   P.gsize = E.gsize;
@@ -1155,10 +1197,10 @@ int wv_engine_enqueue(WvEngine &E, unsigned single_src, unsigned long long timeo
   P.grp = E.grp;
   P.single_src = single_src;
   P.timeout_ns = timeout_ns;
-  wv_schedule(P, E.shape, E.qs_host[0].n, E.qs_host[0].piece != nullptr);
+  wv_schedule(P, E.shape);
   const bool grp = E.shape == WV_GROUP || E.shape == WV_POOL;
-  P.filled = grp || (E.nq == 1u && E.qs_host[0].n > (1u << 18)) ? 1u : 0u;
-  if (grp && cudaMemsetAsync(E.grp, 0, WV_GRP_WORDS * 4, st) != cudaSuccess) return -5;
+  P.filled = E.nq == 1u && (grp || E.qs_host[0].n > (1u << 18)) ? 1u : 0u;
+  if (grp && cudaMemsetAsync(E.grp, 0, (size_t)E.groups * WV_GRP_WORDS * 4, st) != cudaSuccess) return -5;
   if (P.filled)
     wave_fill<<<1184, 256, 0, st>>>(E.qs, single_src,
                                     E.flt ? ADDS_INF_F32_BITSV : ADDS_INF_I32_BITS);

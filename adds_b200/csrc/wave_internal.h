@@ -35,6 +35,8 @@ struct WvQuery {
   unsigned src;
   float delta;        /* first step of the near threshold, in distance units   */
   unsigned np;        /* pieces                                               */
+  unsigned hops;      /* groups: hops between two exchanges                   */
+  unsigned grow;      /* groups: the threshold's step may widen               */
   unsigned long long m;
 };
 
@@ -55,14 +57,14 @@ struct WvStat {
 
 struct WvParams {
   const WvQuery *qs;
-  const unsigned *order;  /* largest first; NULL = 0..nq-1                     */
+  const unsigned *order;  /* the queries, largest first                        */
+  const unsigned *qoff;   /* [groups + 1]: each group's share of the order; null:
+                             one group, or (one CTA per query) all of it       */
   unsigned nq, groups, gsize; /* queries, groups of CTAs, CTAs of one        */
   const WvArea *area;     /* [groups * gsize]                                  */
   void *ws;
   WvStat *st;
   unsigned *grp;          /* a group's notes, two sets; cleared before a launch */
-  unsigned grow;          /* the threshold's step may widen                    */
-  unsigned hops;          /* hops between two exchanges of a group             */
   unsigned single_src;    /* overrides query 0's source when != ~0             */
   unsigned filled;        /* the distances hold INF and the source already     */
   unsigned low;           /* a frontier below this takes more far entries      */
@@ -87,6 +89,7 @@ struct WvEngine {
   WvStat *st = nullptr;
   WvStat *st_host = nullptr; /* pinned                                         */
   std::vector<WvQuery> qs_host;
+  bool shares = false;  /* order is split over the groups                       */
   bool has_set = false; /* room for settled lists                             */
   size_t bytes = 0;
 };
@@ -103,7 +106,8 @@ struct WvEngine {
  * variant (needed before its first launch), the schedule's parameters for P's
  * group size, a launch, and a CTA's frontier entries in shared memory */
 cudaError_t wv_prepare(bool flt, int shape, int *ctas_per_sm);
-void wv_schedule(WvParams &P, int shape, unsigned n, bool pieces);
+void wv_schedule(WvParams &P, int shape);
+void wv_query_schedule(WvQuery &q, int shape);
 cudaError_t wv_launch(const WvParams &P, bool flt, int shape, cudaStream_t st);
 unsigned wv_near(int shape);
 

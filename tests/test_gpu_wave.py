@@ -205,3 +205,36 @@ def test_pooled_after_weight_update():
             d, _ = dg.sssp(9, A.default_opts(timeout_ms=10000, wave=POOL, light_heavy=lh))
             assert np.array_equal(d, O.dijkstra(n, 9)[0])
     dg.close()
+
+
+@pytest.mark.parametrize("nq,ctas", [(1, 0), (2, 0), (7, 20), (40, 0), (40, 1), (150, 3)])
+@pytest.mark.parametrize("wtype", [G.I32, G.F32])
+def test_batches_in_groups(nq, ctas, wtype):
+    """Groups of CTAs that take several queries each, dense and sparse graphs,
+    with new sources and new weights between runs."""
+    rng = np.random.default_rng(nq + ctas)
+    w = dict(wtype=wtype, w_lo=1, w_hi=100)
+    gs = [G.rmat(11, 16, seed=1, **w), G.erdos_renyi(3000, 8, seed=2, **w),
+          G.erdos_renyi(50, 6, seed=3, **w), G.rmat(13, 12, seed=4, **w),
+          G.grid(50, 40, 0.02, 8, seed=5, **w)]
+    dgs = [A.Graph.from_csr(g) for g in gs]
+    pick = [int(x) for x in rng.integers(0, len(gs), size=nq)]
+    for kw in ({}, dict(wave=POOL, light_heavy=1, group_ctas=ctas), dict(wave=GROUP, group_ctas=ctas)):
+        b = A.Batch([dgs[p] for p in pick], [0] * nq, A.default_opts(timeout_ms=20000, **kw))
+        for turn in range(2):
+            srcs = [int(rng.integers(0, gs[p].n)) for p in pick]
+            b.set_sources(srcs)
+            if turn == 1:
+                for i, g in enumerate(gs):
+                    v = rng.integers(1, 50, g.m)
+                    v = v.astype(np.float32).view(np.uint32) if wtype == G.F32 else v.astype(np.uint32)
+                    gs[i] = G.CSR(g.n, g.row, g.dst, v, wtype)
+                    dgs[i].set_weights(v)
+            b.run()
+            st = b.run()
+            assert st["retries"] == 0
+            for q in range(nq):
+                assert np.array_equal(b.dist(q), O.dijkstra(gs[pick[q]], srcs[q])[0]), (kw, turn, q)
+        b.close()
+    for d in dgs:
+        d.close()
