@@ -1388,16 +1388,29 @@ static float wave_delta(const adds_graph *g, int shift, float scale) {
  * heavy edges apart: a hub that is improved again within a bucket relaxes its
  * light edges only.  For graphs with long rows that are large enough for edges
  * rather than hops to count (R-MAT 20 0.85 ms against 1.2 with whole rows,
- * R-MAT 18 0.62 both, R-MAT 16 0.49 against 0.41: the heavy hops are extra);
- * ER 10^6 x 8 1.0 against 0.56. */
-static int wave_layout(adds_graph *g, const Knobs &k, int shift, float scale, const uint2 **edges,
-                       const unsigned **split) {
-  *edges = g->edges;
-  *split = nullptr;
+ * R-MAT 18 0.62 both, R-MAT 16 0.49 against 0.41, all on 148 CTAs: the heavy hops
+ * are extra, and fewer CTAs make edges count sooner); ER 10^6 x 8 1.0 against
+ * 0.56. */
+static int wave_layout(adds_graph *g, const Knobs &k, int shift, float scale, unsigned ctas,
+                       WvQuery *q) {
+  q->edges = g->edges;
+  q->split = nullptr;
+  q->trow = nullptr;
+  q->tedges = nullptr;
   if (k.wave != WV_POOL || k.light_heavy == 0 ||
-      (k.light_heavy == 2 && (g->max_deg <= WV_PIECE || g->n <= (1u << 18))))
+      (k.light_heavy == 2 && (g->max_deg <= WV_PIECE || g->n <= 1771u * ctas)))
     return ADDS_OK;
-  return graph_layout(g, k, shift, scale, edges, split);
+  int rc = graph_layout(g, k, shift, scale, &q->edges, &q->split);
+  /* Heavy edges pulled where that reads less, if edges count at all: R-MAT 21 on
+   * 148 CTAs 1.11 ms against 1.20, R-MAT 22 1.6 against 1.8, R-MAT 20 0.90 against
+   * 0.89; 64 R-MAT 20 queries in groups of 4 18.8 against 21.2. */
+  if (!rc && k.pull && (k.pull == 1 || g->m >= 113000ull * ctas)) {
+    rc = graph_transposed(g);
+    q->trow = g->trow;
+    q->tedges = g->tedges;
+    q->thr = light_threshold(g, shift, scale);
+  }
+  return rc;
 }
 
 static int graph_wave_engine(adds_graph *g, const Knobs &k, int shift, float scale) {
@@ -1406,7 +1419,7 @@ static int graph_wave_engine(adds_graph *g, const Knobs &k, int shift, float sca
   WvQuery q;
   memset(&q, 0, sizeof q);
   q.row = g->row;
-  const int rl = wave_layout(g, k, shift, scale, &q.edges, &q.split);
+  const int rl = wave_layout(g, k, shift, scale, k.group_ctas > 0 ? (unsigned)k.group_ctas : 148u, &q);
   if (rl) return rl;
   q.first = g->wfirst;
   q.piece = g->wpiece;
@@ -1417,9 +1430,11 @@ static int graph_wave_engine(adds_graph *g, const Knobs &k, int shift, float sca
   q.delta = wave_delta(g, shift, scale);
   WvEngine &E = g->weng;
   const unsigned gs = (unsigned)std::max(0, k.group_ctas);
-  if (E.nq == 1 && E.shape == k.wave && E.req_gsize == gs && (E.has_set || !q.split)) {
+  if (E.nq == 1 && E.shape == k.wave && E.req_gsize == gs && (E.has_set || !q.split) &&
+      (E.kernel == WV_PULL || !q.trow)) {
     const WvQuery &h = E.qs_host[0];
-    if (h.delta == q.delta && h.edges == q.edges && h.split == q.split) return ADDS_OK;
+    if (h.delta == q.delta && h.edges == q.edges && h.split == q.split && h.trow == q.trow &&
+        h.thr == q.thr) return ADDS_OK;
     E.qs_host[0] = q;
     wv_query_schedule(E.qs_host[0], k.wave);
     return wv_engine_upload(E, g->stream) ? ADDS_ERR_CUDA : ADDS_OK;
@@ -1544,16 +1559,17 @@ static cudaStream_t pick_stream(const adds_graph *g, const adds_opts *o) {
  *   vertices, where a group's exchanges cost what its width saves (16^2 0.107
  *   against 0.118, 64^2 0.295 against 0.25);
  *   longer rows: ER 4,001 x 8 0.16 against 0.57 (0.29), ER 10^6 x 8 0.56 against
- *   1.7 (0.95), R-MAT 16 0.38 against 0.84 (0.49), R-MAT 20 0.85 against 1.8
- *   (1.15), R-MAT 22 1.7 against 1.9, float 2.0 against 2.4; R-MAT 23 2.55 against
- *   2.25: from there the phase engine's pull phases win, which relax half the
- *   edges. */
+ *   1.7 (0.95), ER 8 x 10^6 x 16 2.3 against 4.4, R-MAT 16 0.40 against 0.84
+ *   (0.49), R-MAT 20 0.89 against 1.8 (1.15), R-MAT 22 1.6 against 2.0, float 1.9
+ *   against 2.4, R-MAT 23 2.3 against 2.4 with weights up to 1,000, 1.7 against 2.2
+ *   up to 10; R-MAT 24 4.5 against 4.2 up to 10,000, 3.6 both up to 1,000: from
+ *   2^27 edges on, graphs with long rows stay with the phase engine. */
 static int auto_wave(const adds_graph *g, const adds_opts *o) {
   if (g->wave_off || g->trace_cap || !schedule_auto(o)) return -1;
   if (g->tuned) return g->tuned_opts.wave > 0 ? g->tuned_opts.wave - 1 : -1;
   if (g->avg_deg < 6.0 && g->m < (1ull << 31)) return g->n < 4096u ? WV_WIDE : WV_GROUP;
   if (g->n < 32768u && g->max_deg <= WV_PIECE) return WV_GROUP; /* ER 4,001 x 8: 0.15, pooled 0.18 */
-  return g->m < 100000000ull ? WV_POOL : -1;
+  return g->m < (g->max_deg <= WV_PIECE ? 1ull << 29 : 1ull << 27) ? WV_POOL : -1;
 }
 
 /* Enqueues one solve; no host synchronisation.  Each solve records four
@@ -1915,7 +1931,7 @@ static int batch_wave_engine(adds_batch *b) {
     WvQuery q;
     memset(&q, 0, sizeof q);
     q.row = g->row;
-    const int rl = wave_layout(g, b->kn, b->shifts[i], b->scales[i], &q.edges, &q.split);
+    const int rl = wave_layout(g, b->kn, b->shifts[i], b->scales[i], b->wave_group, &q);
     if (rl) return rl;
     q.first = g->wfirst;
     q.piece = g->wpiece;
@@ -2041,13 +2057,13 @@ extern "C" int adds_batch_create(adds_graph *const *graphs, const uint32_t *srcs
      * SMs each 2.0, the asynchronous engine 4.7), else four queries to an SM (128
      * grids x 16 sources 7.3 ms against 98).  Others: groups of at least four SMs,
      * which take the queries one after another (192 ER graphs and 64 sources on
-     * R-MAT 20 in groups of 1, 2, 4, 6, 9, 18: 38, 23.5, 21.9, 22.3, 22.8, 26.4 ms;
-     * phase engine 27.6). */
+     * R-MAT 20 in groups of 1, 2, 4, 6, 9, 18: 38, 23.5, 21.9, 22.3, 22.8, 26.4 ms
+     * before pulls, 18.8 in groups of 4 with them; phase engine 27.6). */
     if (b->kn.wave < 0 && schedule_auto(opts)) {
       bool sparse = true, fits = true;
       for (adds_graph *g : b->ugraph) {
         sparse = sparse && g->avg_deg < 6.0;
-        fits = fits && g->m < 100000000ull;
+        fits = fits && g->m < (1ull << 27);
       }
       if (sparse) b->kn.wave = nq <= 37u ? WV_GROUP : (nq <= 148u ? WV_WIDE : WV_CTA);
       else if (fits) b->kn.wave = WV_POOL;
@@ -2140,13 +2156,10 @@ static int batch_relayout(adds_batch *b) {
     bool moved = false;
     for (size_t i = 0; i < b->qgraph.size(); ++i) {
       WvQuery &q = b->weng.qs_host[i];
-      const uint2 *edges;
-      const unsigned *split;
-      const int rc = wave_layout(b->qgraph[i], b->kn, b->shifts[i], b->scales[i], &edges, &split);
+      const WvQuery was = q;
+      const int rc = wave_layout(b->qgraph[i], b->kn, b->shifts[i], b->scales[i], b->wave_group, &q);
       if (rc) return rc;
-      moved = moved || q.edges != edges || q.split != split;
-      q.edges = edges;
-      q.split = split;
+      moved = moved || q.edges != was.edges || q.split != was.split || q.trow != was.trow;
     }
     for (size_t i = 0; i < b->ugraph.size(); ++i) b->wversions[i] = b->ugraph[i]->wversion;
     return moved && wv_engine_upload(b->weng, b->stream) ? ADDS_ERR_CUDA : ADDS_OK;

@@ -89,7 +89,9 @@ struct __align__(16) Ctr {
   unsigned pad[3];
 };
 
-template <int BLOCK, int NS, bool POOL>
+#define PULL_V 4u /* vertices a thread takes per chunk of a pull              */
+
+template <int BLOCK, int NS, int PL>
 struct WSmem {
   uint2 nb[2][NS];  /* frontier entries (v, d): this hop's, the next          */
   Ctr ctr[3];
@@ -100,8 +102,13 @@ struct WSmem {
   unsigned q, r0;
   unsigned pre[WV_MAX_GROUP]; /* inclusive frontier counts of the CTAs        */
   /* POOL: the rows being relaxed by the whole CTA, and their edge offsets    */
-  static constexpr int PB = POOL ? BLOCK : 1;
+  static constexpr int PB = PL == 2 ? PULL_V * BLOCK : (PL == 1 ? BLOCK : 1);
   unsigned it_r0[PB], it_d[PB], it_off[PB], wsum[32];
+  /* POOL with in-edges: the settled entries' heavy edges and in-edges (an
+   * entry that settles twice counts twice), and their smallest distance; the
+   * group's totals                                                           */
+  unsigned long long heavy, into, t_heavy, t_into;
+  unsigned smin, t_smin, t_set, gsize;
 };
 
 /* lists of one CTA in HBM */
@@ -151,10 +158,13 @@ __device__ __forceinline__ uint4 ld_note(const ulonglong2 *p) {
 
 /* GRP: several CTAs per query.  POOL: a CTA pools the edges of its entries
  * over all its threads (graphs whose rows differ much in length); without it
- * each warp relaxes its own entries. */
-template <bool FLT, int BLOCK, int NS, bool GRP, bool POOL>
+ * each warp relaxes its own entries.  PULL: heavy hops may be pulls (PL 0: none
+ * of these, 1: POOL, 2: both; the code alone costs the pooled hop 5 % in
+ * registers). */
+template <bool FLT, int BLOCK, int NS, bool GRP, int PL>
 struct Wave {
-  using Smem = WSmem<BLOCK, NS, POOL>;
+  static constexpr bool POOL = PL >= 1, PULL = PL == 2;
+  using Smem = WSmem<BLOCK, NS, PL>;
 
   /* one thread's state over a query; all but the counts is uniform */
   struct State {
@@ -164,6 +174,7 @@ struct Wave {
     const unsigned *first; /* long rows: a row's first piece, the pieces       */
     const uint4 *piece;
     const unsigned *split; /* light edges at the start of each row, or null    */
+    const unsigned *trow;  /* in-edges, or null: heavy hops may be pulls        */
     unsigned *dist;
     unsigned n, np;
     unsigned T;    /* near threshold (distance word)                          */
@@ -174,6 +185,10 @@ struct Wave {
     unsigned npush, nstale;
     unsigned long long nedge;
   };
+  static constexpr unsigned SUB = BLOCK < 256 ? BLOCK : 256; /* a part of a pooled CTA */
+  static __device__ __forceinline__ void bar_part(unsigned part) {
+    asm volatile("bar.sync %0, %1;" ::"r"(part + 1u), "r"(SUB) : "memory");
+  }
   static __device__ __forceinline__ unsigned next3(unsigned i) { return i == 2u ? 0u : i + 1u; }
 
   static __device__ __forceinline__ uint2 entry(const Smem &S, const State &w, unsigned i) {
@@ -185,14 +200,50 @@ struct Wave {
     else if (i - NS < w.L.ncap) __stcg(w.L.over + (size_t)buf * w.L.ncap + (i - NS), e);
   }
 
+  /* Appends the lanes' improvements (v, nd) in keep to frontier buffer buf and
+   * the far list: one reservation per list and warp.  Returns what lane 0 is
+   * to count. */
+  template <int U>
+  static __device__ __forceinline__ unsigned push(Smem &S, const State &w, Ctr &C, unsigned buf,
+                                                  const unsigned (&v)[U], const unsigned (&nd)[U],
+                                                  unsigned keep) {
+    const unsigned lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    unsigned bn[U], bf[U], cn = 0, cf = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool p = (keep >> u) & 1u, nr = nd[u] < w.T;
+      bn[u] = __ballot_sync(0xFFFFFFFFu, p && nr);
+      bf[u] = __ballot_sync(0xFFFFFFFFu, p && !nr);
+      cn += __popc(bn[u]);
+      cf += __popc(bf[u]);
+    }
+    if ((cn | cf) == 0u) return 0u;
+    unsigned at = 0;
+    if (lane < 2u) at = atomicAdd(lane ? &C.far_new : &C.near_cnt, lane ? cf : cn);
+    unsigned pn = __shfl_sync(0xFFFFFFFFu, at, 0);
+    unsigned pf = __shfl_sync(0xFFFFFFFFu, at, 1) + w.F;
+    if (pn + cn > NS + w.L.ncap || pf + cf > w.L.fcap) C.stop = WV_ERR_OVERFLOW;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint2 e = make_uint2(v[u], nd[u]);
+      if ((bn[u] >> lane) & 1u) put(S, w, buf, pn + __popc(bn[u] & lt), e);
+      if ((bf[u] >> lane) & 1u) {
+        const unsigned i = pf + __popc(bf[u] & lt);
+        if (i < w.L.fcap) __stcg(w.L.far + i, e);
+      }
+      pn += __popc(bn[u]);
+      pf += __popc(bf[u]);
+    }
+    return lane == 0u ? cn + cf : 0u;
+  }
+
   /* Relaxes the edges ed (those in msk) of each lane from distance words dd
    * and pushes the improvements: one reservation per list and warp. */
   template <int U>
   static __device__ __forceinline__ void relax(Smem &S, State &w, const uint2 (&ed)[U],
                                                const unsigned (&dd)[U], unsigned msk,
                                                bool direct = false) {
-    const unsigned lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-    unsigned nd[U], cur[U], bn[U], bf[U], cn = 0, cf = 0;
+    unsigned nd[U], cur[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       nd[u] = add_word<FLT>(dd[u], ed[u].y);
@@ -210,33 +261,13 @@ struct Wave {
         cur[u] = 0u;
       }
     }
+    unsigned keep = 0, v[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const bool p = nd[u] < cur[u], nr = nd[u] < w.T;
-      bn[u] = __ballot_sync(0xFFFFFFFFu, p && nr);
-      bf[u] = __ballot_sync(0xFFFFFFFFu, p && !nr);
-      cn += __popc(bn[u]);
-      cf += __popc(bf[u]);
+      v[u] = ed[u].x;
+      if (nd[u] < cur[u]) keep |= 1u << u;
     }
-    if ((cn | cf) == 0u) return;
-    Ctr &C = S.ctr[next3(w.ci)];
-    unsigned at = 0;
-    if (lane < 2u) at = atomicAdd(lane ? &C.far_new : &C.near_cnt, lane ? cf : cn);
-    unsigned pn = __shfl_sync(0xFFFFFFFFu, at, 0);
-    unsigned pf = __shfl_sync(0xFFFFFFFFu, at, 1) + w.F;
-    if (pn + cn > NS + w.L.ncap || pf + cf > w.L.fcap) C.stop = WV_ERR_OVERFLOW;
-    if (lane == 0) w.npush += cn + cf;
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint2 e = make_uint2(ed[u].x, nd[u]);
-      if ((bn[u] >> lane) & 1u) put(S, w, w.cur ^ 1u, pn + __popc(bn[u] & lt), e);
-      if ((bf[u] >> lane) & 1u) {
-        const unsigned i = pf + __popc(bf[u] & lt);
-        if (i < w.L.fcap) __stcg(w.L.far + i, e);
-      }
-      pn += __popc(bn[u]);
-      pf += __popc(bf[u]);
-    }
+    w.npush += push<U>(S, w, S.ctr[next3(w.ci)], w.cur ^ 1u, v, nd, keep);
   }
 
   /* a lane's entry: its row (or its piece of a long row: ids from n up), and
@@ -391,14 +422,136 @@ struct Wave {
     __syncthreads();
   }
 
+  /* The heavy edges of the settled vertices taken from the other side: every
+   * vertex whose distance lies above floor -- the only ones they can improve,
+   * floor being the smallest settled distance plus the smallest heavy weight --
+   * takes the minimum over its in-edges.  Every candidate is a path's length, a
+   * vertex is written by its thread only, and an improvement that a neighbour
+   * misses in this hop reaches it when the improved vertex is popped.
+   * Improvements join the frontier that is waiting, and the far list.  For
+   * large buckets of graphs whose hubs settle early: R-MAT 22 relaxes 1.3 times
+   * its edges without, 0.54 with (1.8 against 1.6 ms; float 2.05 against 1.92). */
+  static __device__ __noinline__ unsigned pull(Smem &S, State w, const uint2 *tedges,
+                                               unsigned floor, unsigned &edges) {
+    constexpr int U = 4, V = PULL_V;
+    const unsigned part = threadIdx.x / SUB, tid = threadIdx.x % SUB, lane = tid & 31u;
+    const unsigned warp = tid >> 5, nparts = BLOCK / SUB;
+    const unsigned G = S.gsize, rank = blockIdx.x % G;
+    unsigned *const it_r0 = S.it_r0 + part * SUB * V, *const it_b = S.it_d + part * SUB * V;
+    unsigned *const it_off = S.it_off + part * SUB * V, *const wsum = S.wsum + part * (SUB / 32u);
+    const bool vec = ((reinterpret_cast<unsigned long long>(w.dist) |
+                       reinterpret_cast<unsigned long long>(w.trow)) & 15ull) == 0ull;
+    unsigned npush = 0, nedge = 0;
+    const unsigned long long step = (unsigned long long)G * nparts * SUB * V;
+    for (unsigned long long c0 = ((unsigned long long)rank * nparts + part) * SUB * V; c0 < w.n;
+         c0 += step) {
+      const unsigned long long v0 = c0 + tid * V;
+      unsigned d[V], rb[V + 1];
+      if (vec && v0 + V <= w.n) {
+        const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(w.dist + v0));
+        const uint4 r = __ldg(reinterpret_cast<const uint4 *>(w.trow + v0));
+        d[0] = x.x; d[1] = x.y; d[2] = x.z; d[3] = x.w;
+        rb[0] = r.x; rb[1] = r.y; rb[2] = r.z; rb[3] = r.w;
+        rb[4] = __ldg(w.trow + v0 + 4);
+      } else {
+#pragma unroll
+        for (int j = 0; j <= V; ++j) {
+          if (j < V) d[j] = v0 + j < w.n ? __ldcg(w.dist + v0 + j) : 0u;
+          rb[j] = v0 + j <= w.n ? __ldg(w.trow + v0 + j) : 0u;
+        }
+      }
+      unsigned sum = 0;
+#pragma unroll
+      for (int j = 0; j < V; ++j)
+        if (v0 + j < w.n && d[j] > floor) sum += rb[j + 1] - rb[j];
+      unsigned off = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xFFFFFFFFu, off, o);
+        if (lane >= (unsigned)o) off += y;
+      }
+      if (lane == 31u) wsum[warp] = off;
+      bar_part(part);
+      unsigned ws = lane < SUB / 32u ? wsum[lane] : 0u;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xFFFFFFFFu, ws, o);
+        if (lane >= (unsigned)o) ws += y;
+      }
+      const unsigned E = __shfl_sync(0xFFFFFFFFu, ws, 31);
+      const unsigned wb = __shfl_sync(0xFFFFFFFFu, ws, (warp + 31u) & 31u);
+      unsigned at = off - sum + (warp ? wb : 0u);
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        const unsigned i = tid * V + j;
+        it_r0[i] = rb[j];
+        it_b[i] = d[j]; /* the best so far */
+        it_off[i] = at;
+        if (v0 + j < w.n && d[j] > floor) at += rb[j + 1] - rb[j];
+      }
+      nedge += sum;
+      bar_part(part);
+      const unsigned k = SUB * V;
+      const unsigned run = ((E + SUB / 32u - 1u) / (SUB / 32u) + 31u) & ~31u;
+      const unsigned re = min(E, (warp + 1u) * run);
+      unsigned lo = 0, fin = 0, at0 = 0;
+      for (unsigned e0 = warp * run; e0 < re; e0 += 32u * U) {
+        uint2 e[U];
+        unsigned it[U], cur[U], msk = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const unsigned j = e0 + u * 32u + lane;
+          e[u] = make_uint2(0u, 0u);
+          if (j < re) {
+            if (j >= fin) {
+              unsigned st = 1u;
+              while (lo + st < k && it_off[lo + st] <= j) {
+                lo += st;
+                st <<= 1;
+              }
+              unsigned hi = min(lo + st, k) - 1u;
+              while (lo < hi) {
+                const unsigned mid = (lo + hi + 1u) >> 1;
+                if (it_off[mid] <= j) lo = mid; else hi = mid - 1u;
+              }
+              fin = lo + 1u < k ? it_off[lo + 1u] : E;
+              at0 = it_r0[lo] - it_off[lo];
+            }
+            e[u] = __ldg(tedges + (at0 + j));
+            msk |= 1u << u;
+          }
+          it[u] = lo;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) cur[u] = ((msk >> u) & 1u) ? __ldcg(w.dist + e[u].x) : 0u;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const unsigned cand = add_word<FLT>(cur[u], e[u].y); /* INF + w improves nothing */
+          if (((msk >> u) & 1u) && cand < it_b[it[u]]) atomicMin(&it_b[it[u]], cand);
+        }
+      }
+      bar_part(part);
+      unsigned v[V], nd[V], keep = 0;
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        v[j] = (unsigned)(v0 + j);
+        nd[j] = it_b[tid * V + j];
+        if (v0 + j < w.n && nd[j] < d[j]) {
+          keep |= 1u << j;
+          __stcg(w.dist + v[j], nd[j]);
+        }
+      }
+      npush += push<V>(S, w, S.ctr[w.ci], w.cur, v, nd, keep);
+      bar_part(part);
+    }
+    edges += nedge;
+    return npush;
+  }
+
   /* A hop whose edges are pooled: SUB threads take every (BLOCK / SUB)th entry,
    * scan the row lengths of SUB entries at a time, and every warp walks 32 x U
    * neighbouring edges at a time.  The parts of a CTA meet only at the hop's
    * end, so that one loads entries while another relaxes edges (256 mixed queries 21.9 ms as one part, 21.2 in four). */
-  static constexpr unsigned SUB = BLOCK < 256 ? BLOCK : 256;
-  static __device__ __forceinline__ void bar_part(unsigned part) {
-    asm volatile("bar.sync %0, %1;" ::"r"(part + 1u), "r"(SUB) : "memory");
-  }
   static __device__ __forceinline__ void hop_pool(Smem &S, State &w, unsigned cnt) {
     constexpr int U = 4;
     constexpr unsigned PARTS = BLOCK / SUB;
@@ -418,6 +571,21 @@ struct Wave {
         unsigned at = 0;
         if (lane == 0) at = atomicAdd(&S.ctr[next3(w.ci)].set_new, (unsigned)__popc(sb));
         at = __shfl_sync(0xFFFFFFFFu, at, 0) + w.H + __popc(sb & lt);
+        if (PULL && w.trow) { /* what a push and a pull of these heavy edges would read */
+          unsigned hv = 0, in = 0;
+          if (set) {
+            hv = __ldg(w.row + x.x + 1) - __ldg(w.row + x.x) - __ldg(w.split + x.x);
+            in = __ldg(w.trow + x.x + 1) - __ldg(w.trow + x.x);
+          }
+          hv = __reduce_add_sync(0xFFFFFFFFu, hv);
+          in = __reduce_add_sync(0xFFFFFFFFu, in);
+          const unsigned sm = __reduce_min_sync(0xFFFFFFFFu, set ? x.y : 0xFFFFFFFFu);
+          if (lane == 0) {
+            atomicAdd(&S.heavy, (unsigned long long)hv);
+            atomicAdd(&S.into, (unsigned long long)in);
+            atomicMin(&S.smin, sm);
+          }
+        }
         if (set) {
           if (at < w.L.scap) __stcg(w.L.set + at, x);
           else S.ctr[next3(w.ci)].stop = WV_ERR_OVERFLOW;
@@ -635,8 +803,15 @@ struct Wave {
         reinterpret_cast<ulonglong2 *>(P.grp) + ((size_t)group * 2u + par) * WV_MAX_GROUP;
     ++round;
     const unsigned tag = round << 3; /* low bits: the error, WV_SETTLED */
+    ulonglong2 *const more = reinterpret_cast<ulonglong2 *>(P.grp) +
+                             (size_t)P.groups * 2u * WV_MAX_GROUP +
+                             ((size_t)group * 2u + par) * 2u * WV_MAX_GROUP;
     if (tid < 32u) {
       if (lane == 0) {
+        if (PULL && w.trow && w.H) {
+          __stcg(more + 2u * rank, make_ulonglong2(S.heavy, S.into));
+          __stcg(more + 2u * rank + 1u, make_ulonglong2(w.H, S.smin));
+        }
         __threadfence(); /* what the CTA published, before its note */
         st_note(notes + rank, min(cnt, xcap), w.F, fmin, tag | stop | (w.H ? WV_SETTLED : 0u));
       }
@@ -690,6 +865,30 @@ struct Wave {
 #pragma unroll
       for (unsigned j = 0; j < J; ++j)
         first += __popc(__ballot_sync(0xFFFFFFFFu, j * 32u + lane < G && c[j] <= lo));
+      if (PULL && w.trow && (st & WV_SETTLED) && tot <= P.low) {
+        unsigned long long hv = 0, in = 0;
+        unsigned ns = 0, sm = 0xFFFFFFFFu;
+        for (unsigned r = lane; r < G; r += 32u) {
+          if (!(ld_note(notes + r).w & WV_SETTLED)) continue;
+          const ulonglong2 a = __ldcg(more + 2u * r), b = __ldcg(more + 2u * r + 1u);
+          hv += a.x;
+          in += a.y;
+          ns += (unsigned)b.x;
+          sm = min(sm, (unsigned)b.y);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+          hv += __shfl_down_sync(0xFFFFFFFFu, hv, o);
+          in += __shfl_down_sync(0xFFFFFFFFu, in, o);
+        }
+        ns = __reduce_add_sync(0xFFFFFFFFu, ns);
+        sm = __reduce_min_sync(0xFFFFFFFFu, sm);
+        if (lane == 0) {
+          S.t_heavy = hv;
+          S.t_into = in;
+          S.t_set = ns;
+          S.t_smin = sm;
+        }
+      }
       if (lane == 0) {
         S.tot = Note{tot, far, fm, st};
         S.far_max = fx;
@@ -769,6 +968,7 @@ struct Wave {
       w.first = Q.first;
       w.piece = Q.piece;
       w.split = Q.split;
+      w.trow = PULL ? Q.trow : nullptr;
       w.np = Q.np;
       w.dist = Q.dist;
       w.n = Q.n;
@@ -789,7 +989,12 @@ struct Wave {
         __syncthreads();
         if (tid == 0) __stcg(Q.dist + src, 0u);
       }
-      if (tid == 0) S.nb[0][0] = make_uint2(src, 0u);
+      if (tid == 0) {
+        S.nb[0][0] = make_uint2(src, 0u);
+        S.heavy = S.into = 0ull;
+        S.smin = 0xFFFFFFFFu;
+        S.gsize = P.gsize;
+      }
       __syncthreads();
       float delta = Q.delta;
       w.T = raise_word<FLT>(0u, delta);
@@ -839,6 +1044,7 @@ struct Wave {
          * dealt out before they are relaxed (ER 300,000 x 16 with weights 1 to
          * 10 overflowed the first CTA's list). */
         bool deal = !P.filled;
+        unsigned long long gone = 0; /* in-edges of settled vertices */
         for (;;) {
           /* up to P.hops hops on this CTA's own entries */
           const unsigned hmax = deal ? 0u : Q.hops;
@@ -870,7 +1076,26 @@ struct Wave {
           if (stop != 0u || (t.near_cnt == 0u && t.far_cnt == 0u && !settled)) break;
           const bool few = t.near_cnt <= P.low && !(dealt && t.near_cnt != 0u);
           if (POOL && few && settled) {
-            unsettle(S, w);
+            bool pulled = false;
+            if constexpr (PULL) if (w.trow) {
+              /* in-edges of the vertices that have not settled yet: a pull reads
+               * at most these */
+              gone += S.t_into;
+              const unsigned long long left = Q.m > gone ? Q.m - gone : 0ull;
+              if (S.t_set > Q.n >> 6 && S.t_heavy > left) {
+                unsigned ne = 0;
+                w.npush += pull(S, w, Q.tedges, add_word<FLT>(S.t_smin, Q.thr), ne);
+                w.nedge += ne;
+                w.H = 0u;
+                pulled = deal = true;
+              }
+              __syncthreads(); /* totals and sums are read */
+              if (tid == 0) {
+                S.heavy = S.into = 0ull;
+                S.smin = 0xFFFFFFFFu;
+              }
+            }
+            if (!pulled) unsettle(S, w);
           } else if (few && t.far_cnt != 0u) {
             deal = S.far_max > 256u && (unsigned long long)S.far_max * P.gsize * 2u > 3ull * t.far_cnt;
             if (Q.grow && round - split_at <= 1u) delta *= 1.5f;
@@ -915,10 +1140,10 @@ struct Wave {
   }
 };
 
-template <bool FLT, int BLOCK, int NS, int MINB, bool GRP, bool POOL>
+template <bool FLT, int BLOCK, int NS, int MINB, bool GRP, int PL>
 __global__ void __launch_bounds__(BLOCK, MINB) wave_kernel(const __grid_constant__ WvParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Wave<FLT, BLOCK, NS, GRP, POOL>::run(P, *reinterpret_cast<WSmem<BLOCK, NS, POOL> *>(smem_raw));
+  Wave<FLT, BLOCK, NS, GRP, PL>::run(P, *reinterpret_cast<WSmem<BLOCK, NS, PL> *>(smem_raw));
 }
 
 /* INF everywhere and 0 at the source, by the whole GPU */
@@ -929,21 +1154,21 @@ __global__ void wave_fill(const WvQuery *qs, unsigned single_src, unsigned inf) 
     Q.dist[v] = v == src ? 0u : inf;
 }
 
-template <bool FLT, int BLOCK, int NS, int MINB, bool GRP, bool POOL>
+template <bool FLT, int BLOCK, int NS, int MINB, bool GRP, int PL>
 static cudaError_t resident(int *bps) {
-  const int smem = (int)sizeof(WSmem<BLOCK, NS, POOL>);
-  auto *k = wave_kernel<FLT, BLOCK, NS, MINB, GRP, POOL>;
+  const int smem = (int)sizeof(WSmem<BLOCK, NS, PL>);
+  auto *k = wave_kernel<FLT, BLOCK, NS, MINB, GRP, PL>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k, BLOCK, smem);
 }
 
-template <bool FLT, int BLOCK, int NS, int MINB, bool GRP, bool POOL>
+template <bool FLT, int BLOCK, int NS, int MINB, bool GRP, int PL>
 static cudaError_t launch(const WvParams &P, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(P.groups * P.gsize);
   cfg.blockDim = dim3(BLOCK);
-  cfg.dynamicSmemBytes = sizeof(WSmem<BLOCK, NS, POOL>);
+  cfg.dynamicSmemBytes = sizeof(WSmem<BLOCK, NS, PL>);
   cfg.stream = st;
   /* the CTAs of a group wait for each other: all must be resident */
   cudaLaunchAttribute at[1];
@@ -951,23 +1176,24 @@ static cudaError_t launch(const WvParams &P, cudaStream_t st) {
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = GRP ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, wave_kernel<FLT, BLOCK, NS, MINB, GRP, POOL>, P);
+  return cudaLaunchKernelEx(&cfg, wave_kernel<FLT, BLOCK, NS, MINB, GRP, PL>, P);
 }
 
 }  // namespace adds_wave
 
 /* (variant, threads, frontier entries in shared memory, CTAs per SM the
- * registers are sized for, several CTAs per query, pooled edges, entries per
+ * registers are sized for, several CTAs per query, pooled edges and pulls, entries per
  * CTA below which a frontier takes more of the far list).  The batch of 128
  * grids x 16 sources: 256 threads x 4 7.2 ms, x 5 7.6, x 6 8.2, 128 x 10 11.4,
  * 512 x 3 7.8, 1024 x 1 14.5.  Low marks: 32 entries 7.6 ms, 16 7.7, 64 8.0, 0
  * 8.2 there; 4096^2 grid on 148 CTAs 2,500 entries 18.3 ms, 1,000 19.3, 9,500
  * 21.7. */
 #define WV_SHAPES(X)                           \
-  X(WV_CTA, 256, 1024, 4, false, false, 32)    \
-  X(WV_WIDE, 1024, 4096, 1, false, false, 64)  \
-  X(WV_GROUP, 512, 2048, 1, true, false, 16)   \
-  X(WV_POOL, 1024, 2048, 1, true, true, 8)
+  X(WV_CTA, 256, 1024, 4, false, 0, 32)        \
+  X(WV_WIDE, 1024, 4096, 1, false, 0, 64)      \
+  X(WV_GROUP, 512, 2048, 1, true, 0, 16)       \
+  X(WV_POOL, 1024, 2048, 1, true, 1, 8)        \
+  X(WV_PULL, 1024, 2048, 1, true, 2, 8)
 
 static unsigned wv_block(int shape) {
 #define X(s, b, ns, m, g, pl, lo) if (shape == s) return b;
@@ -1024,7 +1250,10 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
   int sms = 0, bps = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
     return -5;
-  const cudaError_t e = wv_prepare(flt, shape, &bps);
+  E.kernel = shape;
+  for (const WvQuery &q : qv)
+    if (shape == WV_POOL && q.trow) E.kernel = WV_PULL;
+  const cudaError_t e = wv_prepare(flt, E.kernel, &bps);
   if (e != cudaSuccess || bps < 1) {
     cudaGetLastError();
     return -9;
@@ -1209,12 +1438,12 @@ int wv_engine_enqueue(WvEngine &E, unsigned single_src, unsigned long long timeo
   wv_schedule(P, E.shape);
   const bool grp = E.shape == WV_GROUP || E.shape == WV_POOL;
   P.filled = E.nq == 1u && (grp || E.qs_host[0].n > (1u << 18)) ? 1u : 0u;
-  if (grp && cudaMemsetAsync(E.grp, 0, (size_t)E.groups * WV_GRP_WORDS * 4, st) != cudaSuccess) return -5;
+  if (grp && cudaMemsetAsync(E.grp, 0, (size_t)E.groups * 2u * 16u * WV_MAX_GROUP, st) != cudaSuccess) return -5;
   if (P.filled)
     wave_fill<<<1184, 256, 0, st>>>(E.qs, single_src,
                                     E.flt ? ADDS_INF_F32_BITSV : ADDS_INF_I32_BITS);
   if (k0 && cudaEventRecordWithFlags(k0, st, fl) != cudaSuccess) return -5;
-  if (wv_launch(P, E.flt, E.shape, st) != cudaSuccess) return -5;
+  if (wv_launch(P, E.flt, E.kernel, st) != cudaSuccess) return -5;
   if (k1 && cudaEventRecordWithFlags(k1, st, fl) != cudaSuccess) return -5;
   if (cudaMemcpyAsync(E.st_host, E.st, sizeof(WvStat), cudaMemcpyDeviceToHost, st) != cudaSuccess)
     return -5;

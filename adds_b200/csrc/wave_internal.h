@@ -19,13 +19,19 @@
 #define WV_SETTLED 4u     /* in a note: the CTA holds settled entries           */
 #define WV_PIECE 512u     /* edges of a long row one entry stands for          */
 #define WV_MAX_GROUP 160u /* CTAs of one group (a multiple of 32)              */
-#define WV_GRP_WORDS (2u * 4u * WV_MAX_GROUP) /* two sets of 16-byte notes     */
+/* a group's two sets of 16-byte notes, and (after all groups' notes) two sets
+ * of 32 bytes on the settled entries */
+#define WV_GRP_WORDS (2u * (4u + 8u) * WV_MAX_GROUP)
 
 struct WvQuery {
   const unsigned *row;
   const uint2 *edges; /* rows in CSR order, or sorted by weight where split is  */
   const unsigned *split; /* WV_POOL: light edges (w < delta) at the start of each
                             row; null: every row is relaxed whole             */
+  /* in-edges (the transposed graph, {tail, weight}) and the smallest heavy
+   * weight's bits, where heavy edges may be pulled; else null                */
+  const unsigned *trow;
+  const uint2 *tedges;
   /* rows of more than WV_PIECE edges: their first piece by vertex, and the
    * pieces {vertex, first edge, edges, 0}; null where no row is that long */
   const unsigned *first;
@@ -35,6 +41,7 @@ struct WvQuery {
   unsigned src;
   float delta;        /* first step of the near threshold, in distance units   */
   unsigned np;        /* pieces                                               */
+  unsigned thr;
   unsigned hops;      /* groups: hops between two exchanges                   */
   unsigned grow;      /* groups: the threshold's step may widen               */
   unsigned long long m;
@@ -79,7 +86,8 @@ struct WvParams {
 struct WvEngine {
   int device = -1;
   bool flt = false;
-  int shape = -1;         /* kernel variant (wave.cu)                          */
+  int shape = -1;         /* variant asked for                                  */
+  int kernel = -1;        /* variant launched (WV_PULL for WV_POOL with in-edges) */
   unsigned nq = 0, groups = 0, gsize = 1, ctas = 0, req_gsize = 0;
   unsigned *grp = nullptr;
   WvQuery *qs = nullptr;
@@ -100,6 +108,7 @@ struct WvEngine {
 #define WV_WIDE 1
 #define WV_GROUP 2
 #define WV_POOL 3
+#define WV_PULL 4 /* WV_POOL with queries that have in-edges                    */
 #define WV_LAST WV_POOL
 
 /* the kernels themselves (noalloc.cu brings its own memory): residency of a

@@ -238,3 +238,41 @@ def test_batches_in_groups(nq, ctas, wtype):
         b.close()
     for d in dgs:
         d.close()
+
+
+@pytest.mark.parametrize("wtype", [G.I32, G.F32])
+@pytest.mark.parametrize("ctas", [1, 4, 148])
+def test_pulled_heavy_hops(wtype, ctas):
+    """Heavy hops from the other side: fewer edges than pushing them, the same
+    distances; sizes that are no multiple of a chunk, vertices without
+    in-edges, unreachable ones, and new weights."""
+    w = dict(wtype=wtype, w_lo=1, w_hi=1000)
+    kw = dict(wave=POOL, light_heavy=1, group_ctas=ctas)
+    r = G.rmat(14, 16, seed=11, **w)
+    src = G.max_degree_vertex(r)
+    push = check(r, [src], pull=-1, **kw)["edges_scanned"]
+    pull = check(r, [src], pull=1, **kw)["edges_scanned"]
+    assert pull < 0.8 * push
+    for shift in (-1, 4, 9) if wtype == G.I32 else (-1, 10, 16):
+        check(G.rmat(11, 24, seed=12, **w), [3, 500], pull=1, delta_shift=shift, **kw)
+        check(G.erdos_renyi(4099, 12, seed=13, **w), [4098], pull=1, delta_shift=shift, **kw)
+    rows = [3000, 700, 0, 5000]
+    check(star(rows, wtype), [0], pull=1, **kw)
+    dg = A.Graph.from_csr(r)
+    for hi in (3, 700):
+        v = np.random.default_rng(hi).integers(0, hi, r.m)
+        v = v.astype(np.float32).view(np.uint32) if wtype == G.F32 else v.astype(np.uint32)
+        dg.set_weights(v)
+        d, _ = dg.sssp(src, A.default_opts(timeout_ms=10000, pull=1, **kw))
+        assert np.array_equal(d, O.dijkstra(G.CSR(r.n, r.row, r.dst, v, wtype), src)[0])
+    dg.close()
+    small = G.rmat(12, 16, seed=14, **w)
+    dg = A.Graph.from_csr(small)
+    b = A.Batch([dg] * 9, list(range(0, 4050, 450)),
+                A.default_opts(timeout_ms=20000, pull=1, **kw))
+    for _ in range(2):
+        b.run()
+    for q in range(9):
+        assert np.array_equal(b.dist(q), O.dijkstra(small, 450 * q)[0])
+    b.close()
+    dg.close()
