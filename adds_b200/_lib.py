@@ -61,8 +61,8 @@ class Opts(C.Structure):
         ("near_far", C.c_int32),
         ("dense_scan", C.c_int32),
         ("pull", C.c_int32),
+        ("reserved", C.c_int32 * 2),
         ("wave", C.c_int32),
-        ("reserved", C.c_int32 * 1),
     ]
 
 

@@ -115,6 +115,7 @@ typedef struct adds_opts {
                             the push.  Keeps a transposed copy of the graph
                             (8 B per edge, built on first use).  0 = auto
                             (on), < 0 = off, 1 = on                         */
+  int32_t reserved[2];
   int32_t wave;          /* solve by a wave kernel (near-far lists, a CTA or a
                             group of CTAs per query) instead of an engine,
                             which takes over where its lists do not suffice:
@@ -123,7 +124,6 @@ typedef struct adds_opts {
                             threads, 2 = a CTA of 1024, 3 = a CTA per SM
                             (plain solves), 4 = a CTA per SM, pooling the
                             edges of its entries (plain solves)              */
-  int32_t reserved[1];
 } adds_opts;
 
 /* Engines.  PHASE settles the buckets in bulk-synchronous phases (light
