@@ -27,7 +27,8 @@ class _SSSP(torch.autograd.Function):
         held = [w.detach().contiguous() for w in weights]
         # the graphs and the batch work on streams of their own: the weights
         # must have been computed, and the zeros written, before they start
-        torch.cuda.current_stream(flat.device).synchronize()
+        for dev in {w.device for w in held if w.is_cuda}:
+            torch.cuda.current_stream(dev).synchronize()
         for g, w in zip(graphs, held):
             g.set_weights(w.data_ptr())
         batch.run()

@@ -31,3 +31,17 @@ def test_forward_waits_for_its_weights(side):
         assert np.array_equal(flat[: g.n].cpu().numpy().view(np.uint32), ref)
     b.close()
     dg.close()
+
+
+def test_forward_takes_host_weights():
+    """Weights that lie in host memory: the distances come back there too."""
+    from adds_b200.autograd import batched_sssp
+    g = G.grid(40, 40, 0.0, 8, wtype=G.F32, seed=3)
+    dg = A.Graph.from_csr(g)
+    b = A.Batch([dg], [5])
+    flat = batched_sssp(b, [dg], [torch.from_numpy(g.w.view(np.float32) * np.float32(2))])
+    n = G.CSR(g.n, g.row, g.dst, (g.w.view(np.float32) * np.float32(2)).view(np.uint32), G.F32)
+    assert flat.device.type == "cpu"
+    assert np.array_equal(flat[: g.n].numpy().view(np.uint32), O.dijkstra(n, 5)[0])
+    b.close()
+    dg.close()
