@@ -146,6 +146,7 @@ SIGNATURES = [
     ("adds_graph_info", C.c_int, [C.c_void_p, C.POINTER(GraphInfo)]),
     ("adds_graph_download", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     ("adds_graph_set_weights", C.c_int, [C.c_void_p, C.c_void_p]),
+    ("adds_graphs_set_weights", C.c_int, [C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.c_uint32]),
     ("adds_graph_save_gr", C.c_int, [C.c_void_p, C.c_char_p]),
     ("adds_graph_free", None, [C.c_void_p]),
     ("adds_graph_generate", C.c_int, [C.POINTER(GenSpec), C.c_int, C.POINTER(C.c_void_p)]),

@@ -13,10 +13,25 @@ Unreached vertices carry no gradient.
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import torch
 
 from . import Batch
+from ._lib import GraphInfo, check, lib
+
+
+def _set_weights(graphs, weights) -> None:
+    """Graph.set_weights of each pair, in one call."""
+    pairs = list(zip(graphs, weights))
+    gs = (C.c_void_p * len(pairs))(*[g.handle.value for g, _ in pairs])
+    ws = (C.c_void_p * len(pairs))(*[w.data_ptr() for _, w in pairs])
+    check(lib().adds_graphs_set_weights(gs, ws, len(pairs)), "adds_graphs_set_weights")
+    info = GraphInfo()
+    for g, _ in pairs:
+        lib().adds_graph_info(g.handle, C.byref(info))
+        g.avg_weight = info.avg_weight
 
 
 class _SSSP(torch.autograd.Function):
@@ -29,8 +44,7 @@ class _SSSP(torch.autograd.Function):
         # must have been computed, and the zeros written, before they start
         for dev in {w.device for w in held if w.is_cuda}:
             torch.cuda.current_stream(dev).synchronize()
-        for g, w in zip(graphs, held):
-            g.set_weights(w.data_ptr())
+        _set_weights(graphs, held)
         batch.run()
         batch.dist_all(flat.data_ptr())
         ctx.batch = batch

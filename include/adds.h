@@ -210,6 +210,11 @@ int adds_graph_download(const adds_graph *g, uint64_t *row_start, uint32_t *dst,
                         void *w);
 /* Overwrites the m edge weights (host or device pointer, CSR order). */
 int adds_graph_set_weights(adds_graph *g, const void *w);
+/* The same for ng graphs at once: graph i takes w[i].  One launch and one wait
+ * where the graphs share a device and the weights lie on it.  If some weights
+ * are invalid the graphs that got them hold them, as after
+ * adds_graph_set_weights. */
+int adds_graphs_set_weights(adds_graph *const *graphs, const void *const *w, uint32_t ng);
 /* Writes the graph as a Galois .gr v1 file (input side of run_all.sh). */
 int adds_graph_save_gr(const adds_graph *g, const char *path);
 void adds_graph_free(adds_graph *g);

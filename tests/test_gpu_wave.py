@@ -276,3 +276,35 @@ def test_pulled_heavy_hops(wtype, ctas):
         assert np.array_equal(b.dist(q), O.dijkstra(small, 450 * q)[0])
     b.close()
     dg.close()
+
+
+@pytest.mark.parametrize("on_gpu", [True, False])
+def test_weights_of_several_graphs_at_once(on_gpu):
+    """Sizes around a tile of 4,096 edges; the mean is the one-graph call's; a
+    graph named twice takes its last weights; invalid weights are refused."""
+    import torch
+    from adds_b200.autograd import _set_weights
+    gs = [G.grid(s, 7, 0.0, 8, wtype=G.F32, seed=s) for s in (2, 40, 157, 158, 900, 6000)]
+    assert any(g.m > 1 << 16 for g in gs)
+    dgs = [A.Graph.from_csr(g) for g in gs]
+    rng = np.random.default_rng(1)
+    ws = [rng.uniform(0.5, 9, g.m).astype(np.float32) for g in gs]
+    ws[1][::5] = -0.0
+    put = (lambda w: torch.from_numpy(w).cuda()) if on_gpu else torch.from_numpy
+    _set_weights(dgs, [put(w) for w in ws])
+    for g, dg, w in zip(gs, dgs, ws):
+        many = dg.avg_weight
+        n = G.CSR(g.n, g.row, g.dst, np.abs(w).view(np.uint32), G.F32)
+        assert np.array_equal(dg.sssp(1)[0], O.dijkstra(n, 1)[0])
+        dg.set_weights(w)
+        assert abs(dg.avg_weight - many) <= 1e-9 * many
+    a, b = ws[4] * 2, ws[4] * 3
+    _set_weights([dgs[4], dgs[0], dgs[4]], [put(a), put(ws[0]), put(b)])
+    n = G.CSR(gs[4].n, gs[4].row, gs[4].dst, b.view(np.uint32), G.F32)
+    assert np.array_equal(dgs[4].sssp(0)[0], O.dijkstra(n, 0)[0])
+    bad = ws[3].copy()
+    bad[-1] = np.nan
+    with pytest.raises(A.AddsError):
+        _set_weights(dgs[2:5], [put(ws[2]), put(bad), put(ws[4])])
+    for d in dgs:
+        d.close()
