@@ -1631,7 +1631,7 @@ static void fill_wave_stats(const WvEngine &E, adds_stats *s) {
   s->phases = t.steps;
   s->batches = t.splits;
   s->ctas = (int32_t)E.ctas;
-  s->launches = 1;
+  s->launches = E.fills ? 2 : 1;
 }
 
 /* error word, reset and counters of whatever ran g's last solves */

@@ -7,9 +7,11 @@
  * synchronises the whole device), or a latency-bound service loop where the
  * implicit synchronisation of cudaMalloc/cudaFree is not acceptable.
  * adds_sssp_noalloc serves them: the caller passes the graph and the output
- * as device arrays it already owns, and all the working memory of the phase
- * engine (bucket page pool, page tables, list tails, split-row records,
- * control block) comes from one file-scope device array of fixed size
+ * as device arrays it already owns, and all the working memory of the wave
+ * kernels (lists, notes, pieces of long rows) and of the phase engine, which
+ * solves where those lists do not suffice (bucket page pool, page tables, list
+ * tails, split-row records, control block), comes from one file-scope device
+ * array of fixed size
  * declared below.  The array exists on every GPU that loads this library, from the
  * moment the library's code is loaded on it until the process exits.
  *

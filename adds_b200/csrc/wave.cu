@@ -1,16 +1,19 @@
 /*
- * wave.cu — near-far SSSP by one CTA or one thread-block cluster per query.
+ * wave.cu — near-far SSSP by one CTA or a group of CTAs per query.
  *
  * Replaces, for thin wave fronts and for batches of many queries, the
  * worklist of the reference (ads_int/wl.h:133-1972) and its relaxation
  * (ads_int/kernel.cu:30-128).  A road network's wave front is a chain of a
  * thousand or more dependent steps; what a step costs is its memory round
- * trips and its barrier, not its bytes.  Here a group that can synchronise in
- * hardware (a CTA, or a cluster of CTAs) runs the chain alone: the frontier
- * lives in shared memory, the step's barrier is bar.sync or
- * barrier.cluster, and nothing is counted, published or claimed through HBM.
- * Many groups run side by side (a batch), one after another from a shared
- * counter, largest first.
+ * trips and its barrier, not its bytes.  Here a CTA runs the chain alone: its
+ * frontier lives in shared memory, a step's barrier is bar.sync, and nothing is
+ * counted, published or claimed through HBM.  A group of CTAs (a CTA per SM for
+ * a plain solve) shares a query: each runs several steps on its own entries,
+ * then they exchange what is left through lists and 16-byte notes in HBM.
+ * (A cluster of 16 CTAs with lists in distributed shared memory was slower: a
+ * barrier.cluster with release costs about 3,500 cycles, and 16 SMs are few.)
+ * Many CTAs or groups run side by side in a batch: single CTAs draw queries
+ * from a shared counter, largest first; groups get shares of equal work.
  *
  * A step pops the frontier's entries (v, d), drops those that a smaller
  * distance has superseded, relaxes the rows and keeps the improvements: those
@@ -48,6 +51,9 @@
  * land in the bucket that is being settled) once per settled vertex, when the
  * frontier has run low.  R-MAT 20 relaxes 1.0 to 1.3 times its edges so, 3.5 to
  * 4 times with whole rows; 0.85 ms against 1.2, and 1.8 on the phase engine.
+ * From some 17 million edges on, heavy hops that would relax more edges than the
+ * in-edges of the vertices above T are pulls (WV_PULL): R-MAT 22 with float
+ * weights 3.9 -> 3.6 ms with its copies, a batch of 8 R-MATs 21.2 -> 19.1.
  * A full hop is bound by scattered requests (gathers 1,900, atomics 2,000, row
  * searches and edge loads 2,500, pushes 1,400 cycles for 4,096 edges of an SM),
  * a small one by its round trips.
@@ -1438,6 +1444,7 @@ int wv_engine_enqueue(WvEngine &E, unsigned single_src, unsigned long long timeo
   wv_schedule(P, E.shape);
   const bool grp = E.shape == WV_GROUP || E.shape == WV_POOL;
   P.filled = E.nq == 1u && (grp || E.qs_host[0].n > (1u << 18)) ? 1u : 0u;
+  E.fills = P.filled != 0u;
   if (grp && cudaMemsetAsync(E.grp, 0, (size_t)E.groups * 2u * 16u * WV_MAX_GROUP, st) != cudaSuccess) return -5;
   if (P.filled)
     wave_fill<<<1184, 256, 0, st>>>(E.qs, single_src,

@@ -1,7 +1,7 @@
 /*
  * wave_internal.h — device data layout of the wave kernels (wave.cu).
  *
- * One group (a CTA, or a thread-block cluster) solves one query with two
+ * One group (a CTA, or several that exchange) solves one query with two
  * kinds of lists: the frontier of the current step, kept in shared memory
  * with an overflow area in HBM, and a far list per CTA in HBM.  No page
  * pool, no bucket ring, no barrier through memory.
@@ -98,6 +98,7 @@ struct WvEngine {
   WvStat *st_host = nullptr; /* pinned                                         */
   std::vector<WvQuery> qs_host;
   bool shares = false;  /* order is split over the groups                       */
+  bool fills = false;   /* the last launch was preceded by the fill kernel     */
   bool has_set = false; /* room for settled lists                             */
   size_t bytes = 0;
 };

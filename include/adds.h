@@ -89,7 +89,8 @@ typedef struct adds_opts {
                             512; phase engine 256, 512 or 1024; 0 = auto       */
   int32_t greed;         /* async engine: a claim takes avail / (CTAs >> greed)
                             entries; <0 = auto                                 */
-  int32_t engine;        /* ADDS_ENGINE_*: 0 = auto (phase)                      */
+  int32_t engine;        /* ADDS_ENGINE_*: 0 = auto (the wave kernels, see wave,
+                            or the phase engine)                              */
   int32_t group_ctas;    /* phase engine: CTAs that solve one query together
                             (batches: the group size; plain solves: the CTAs
                             launched, fewer making each phase's barrier
@@ -121,9 +122,9 @@ typedef struct adds_opts {
                             which takes over where its lists do not suffice:
                             0 = auto (only where every knob of the schedule
                             is automatic too), < 0 = no, 1 = a CTA of 256
-                            threads, 2 = a CTA of 1024, 3 = a CTA per SM
-                            (plain solves), 4 = a CTA per SM, pooling the
-                            edges of its entries (plain solves)              */
+                            threads, 2 = a CTA of 1024, 3 = a CTA per SM, 4 =
+                            a CTA per SM that pools the edges of its entries
+                            (in a batch 3 and 4 split the SMs into groups)   */
 } adds_opts;
 
 /* Engines.  PHASE settles the buckets in bulk-synchronous phases (light
@@ -141,7 +142,8 @@ typedef struct adds_stats {
   uint64_t items_stale;     /* popped entries skipped as superseded            */
   uint64_t edges_scanned;   /* edges of expanded vertices (float work count)   */
   uint64_t pushes;          /* queue entries pushed                            */
-  uint64_t batches;         /* CTA-level pops (phase engine: frontier chunks)  */
+  uint64_t batches;         /* CTA-level pops (phase engine: frontier chunks;
+                               wave kernels: splits of the far list)         */
   uint64_t hub_chunks;      /* split row chunks processed                      */
   uint64_t hub_stale;       /* of which skipped (row's vertex had improved)    */
   uint64_t local_batches;   /* batches a CTA took from its own pushes          */
@@ -163,11 +165,14 @@ typedef struct adds_stats {
   int32_t engine;           /* ADDS_ENGINE_ASYNC or ADDS_ENGINE_PHASE: what ran,
                                or what a wave kernel stood in for            */
   int32_t launches;         /* kernel launches per solve: async 2 (init, solver);
+                               wave kernel 2 (fill, solver; small ones 1);
                                phase 1, or 5 with pull phases possible (phase,
                                pull, phase, pull, phase; unused ones return at
                                once)                                         */
   int32_t reserved[3];
-  uint64_t phases;          /* phase engine: phases decided (solo included)    */
+  uint64_t phases;          /* phase engine: phases decided (solo included);
+                               wave kernels: exchanges of a group, or a CTA's
+                               hops                                          */
   uint64_t solo_phases;     /* phase engine: phases run by one CTA             */
   uint64_t repushes;        /* phase engine: far-slot entries moved on         */
 } adds_stats;
