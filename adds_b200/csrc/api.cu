@@ -1700,6 +1700,28 @@ static int auto_wave(const adds_graph *g, const adds_opts *o) {
   return g->m < (g->max_deg <= WV_PIECE ? 1ull << 29 : 1ull << 27) ? WV_POOL : -1;
 }
 
+/* The bucket of a pooled wave kernel that relaxes light and heavy edges apart,
+ * no narrower than auto_shift's.  Where rows are long, the 4 avg_w / degree of
+ * auto_shift is too narrow above a degree of 8: the heavy edges that a wide
+ * bucket saves for later are most of the rows at any of these degrees.  Best
+ * over degrees 8 to 64, scales 17 to 22 and seven weight ranges: 0.44 of a
+ * mean weight, a quarter once the heavy edges are pulled, less from some 90
+ * million edges on (R-MAT 18 x 16 0.68 -> 0.58 ms, 18 x 64 1.35 -> 0.98, 20 x 16 0.99
+ * -> 0.94, 20 x 32 1.55 -> 1.10, 21 x 32 1.73 -> 1.48 with weights up to 10,000; up
+ * to 10 and 100 it saves more, for floats less: 19 x 32 with a = 0.7 loses 6 %,
+ * 22 x 24 lost 13 % at a quarter).  Integer weights have one added, so that
+ * few-valued ones have light edges.  Not below 664
+ * vertices a CTA, where the rows are relaxed whole and there is little to
+ * settle (R-MAT 16 0.34 -> 0.36; R-MAT 17 0.50 -> 0.48), nor without long rows (ER
+ * 10^6 x 32 0.73 at auto_shift's 2^9, 1.3 at 2^11). */
+static int pooled_shift(const adds_graph *g, int shift) {
+  constexpr unsigned ctas = 148;
+  if (g->max_deg <= WV_PIECE || g->n <= 664u * ctas) return shift;
+  const double c = g->m >= 610000ull * ctas ? 0.175 : g->m >= 113000ull * ctas ? 0.25 : 0.44;
+  const double keys = g->wt == ADDS_F32 ? c * 65536.0 : c * g->avg_w + 1.0;
+  return std::max(shift, std::min(31, (int)lround(log2(keys))));
+}
+
 /* Enqueues one solve; no host synchronisation.  Each solve records four
  * events (start, solver start, solver end, end) in the graph's ring. */
 static int sssp_enqueue(adds_graph *g, uint32_t src, const adds_opts *opts) {
@@ -1707,7 +1729,10 @@ static int sssp_enqueue(adds_graph *g, uint32_t src, const adds_opts *opts) {
   float scale;
   Knobs k;
   resolve(g, opts, &k, &shift, &scale);
-  if (k.wave < 0) k.wave = auto_wave(g, opts);
+  if (k.wave < 0) {
+    k.wave = auto_wave(g, opts);
+    if (k.wave == WV_POOL && !g->tuned) shift = pooled_shift(g, shift);
+  }
   if (g->wave_off) k.wave = -1;
   const bool phase = k.engine == ADDS_ENGINE_PHASE, wave = k.wave >= 0;
   int rc = ADDS_OK;

@@ -308,3 +308,25 @@ def test_weights_of_several_graphs_at_once(on_gpu):
         _set_weights(dgs[2:5], [put(ws[2]), put(bad), put(ws[4])])
     for d in dgs:
         d.close()
+
+
+@pytest.mark.parametrize("wt,hi", [(0, 1), (0, 9), (0, 10000), (1, 1.0)])
+@pytest.mark.parametrize("n", [98272, 98273, 300000])
+def test_width_of_pooled_buckets(n, wt, hi):
+    """Around the line from which long rows take a wider bucket, against the
+    phase engine; weights all 1 and few-valued ones included."""
+    rng = np.random.default_rng(n)
+    m = 12 * n
+    dst = rng.integers(0, n, m).astype(np.uint32)
+    src = np.where(rng.random(m) < 0.05, 7, rng.integers(0, n, m)).astype(np.int64)
+    w = rng.integers(1, hi + 1, m).astype(np.uint32) if wt == 0 else rng.random(m).astype(np.float32).view(np.uint32)
+    order = np.argsort(src, kind="stable")
+    row = np.zeros(n + 1, np.uint64)
+    np.cumsum(np.bincount(src, minlength=n), out=row[1:])
+    dg = A.Graph.from_csr(G.CSR(n, row, dst[order], w[order], wt))
+    a, sa = dg.sssp(7)
+    b, sb = dg.sssp(7, A.default_opts(engine=2))
+    assert np.array_equal(a, b)
+    assert sa["delta_shift"] >= sb["delta_shift"]
+    assert n > 98272 or sa["delta_shift"] == sb["delta_shift"]
+    dg.close()
