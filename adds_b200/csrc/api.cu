@@ -386,6 +386,17 @@ static void fill_stats(const Engine &E, const EngParams &P, adds_stats *s) {
 
 /* ------------------------------------------------------------------------ */
 /* graphs                                                                     */
+
+/* Where the light edges of each sorted row end, for one bucket width.  A graph's
+ * plain solves and each of its batches own one: their widths differ, they may
+ * run at the same time, and a pull relies on its solve's own threshold. */
+struct Split {
+  unsigned *at = nullptr; /* light-edge count per row                       */
+  unsigned thr = 0;       /* ... of weights below this (weight bits)        */
+  unsigned long long wversion = 0; /* ... of these weights                  */
+  bool valid = false;
+};
+
 struct adds_graph {
   int device = 0;
   adds_wtype wt = ADDS_I32;
@@ -395,9 +406,8 @@ struct adds_graph {
   uint2 *edges = nullptr;
   unsigned *dist = nullptr;
   uint2 *sedges = nullptr;     /* rows sorted by weight (light edges first)   */
-  unsigned *split = nullptr;   /* light-edge count per row for split_thr      */
-  unsigned split_thr = 0;
-  bool sorted_valid = false, split_valid = false;
+  bool sorted_valid = false;
+  Split split;                 /* the plain solves' one                       */
   unsigned *trow = nullptr;    /* in-edge CSR (pull phases): n+1 offsets      */
   uint2 *tedges = nullptr;     /* {tail vertex, weight bits} per in-edge      */
   bool trans_valid = false;
@@ -629,7 +639,7 @@ extern "C" void adds_graph_free(adds_graph *g) {
   if (g->edges) cudaFree(g->edges);
   if (g->dist) cudaFree(g->dist);
   if (g->sedges) cudaFree(g->sedges);
-  if (g->split) cudaFree(g->split);
+  if (g->split.at) cudaFree(g->split.at);
   if (g->trow) cudaFree(g->trow);
   if (g->tedges) cudaFree(g->tedges);
   if (g->wfirst) cudaFree(g->wfirst);
@@ -1009,8 +1019,8 @@ extern "C" int adds_graph_set_weights(adds_graph *g, const void *w) {
   double sw;
   memcpy(&sw, h + 2, 8);
   g->avg_w = sw / ns;
-  g->sorted_valid = g->split_valid = false; /* the weight order changed */
-  g->trans_valid = false;                   /* the in-edges carry weights */
+  g->sorted_valid = false; /* the weight order changed */
+  g->trans_valid = false;  /* the in-edges carry weights */
   ++g->wversion;
   return ADDS_OK;
 }
@@ -1084,7 +1094,7 @@ extern "C" int adds_graphs_set_weights(adds_graph *const *graphs, const void *co
       continue;
     }
     g->avg_w = j.sum / j.ns;
-    g->sorted_valid = g->split_valid = false;
+    g->sorted_valid = false;
     g->trans_valid = false;
     ++g->wversion;
   }
@@ -1271,7 +1281,6 @@ static int graph_sorted(adds_graph *g) {
     g->sort_tmp_bytes = 0;
   }
   g->sorted_valid = true;
-  g->split_valid = false;
   return ADDS_OK;
 }
 
@@ -1286,37 +1295,43 @@ static unsigned light_threshold(const adds_graph *g, int shift, float scale) {
   return b;
 }
 
-static int graph_split(adds_graph *g, unsigned thr) {
+/* S for threshold thr and g's present weights.  *rebuilt: work was queued on
+ * the graph's stream. */
+static int graph_split(adds_graph *g, Split &S, unsigned thr, bool *rebuilt) {
+  *rebuilt = !g->sorted_valid;
   int rc = graph_sorted(g);
   if (rc) return rc;
-  if (g->split_valid && g->split_thr == thr) return ADDS_OK;
-  if (!g->split) {
-    CK(cudaMalloc(&g->split, ((size_t)g->n ? g->n : 1) * 4));
-    g->bytes += (size_t)g->n * 4;
+  if (S.valid && S.thr == thr && S.wversion == g->wversion) return ADDS_OK;
+  *rebuilt = true;
+  S.valid = false;
+  if (!S.at) {
+    CK(cudaMalloc(&S.at, ((size_t)g->n ? g->n : 1) * 4));
+    if (&S == &g->split) g->bytes += (size_t)g->n * 4;
   }
-  k_split<<<592, 256, 0, g->stream>>>(g->row, g->sedges, g->n, thr, g->split);
+  k_split<<<592, 256, 0, g->stream>>>(g->row, g->sedges, g->n, thr, S.at);
   CK(cudaGetLastError());
-  g->split_thr = thr;
-  g->split_valid = true;
+  S.thr = thr;
+  S.wversion = g->wversion;
+  S.valid = true;
   return ADDS_OK;
 }
 
-/* edge array and light counts the engine should use for this graph */
-static int graph_layout(adds_graph *g, const Knobs &k, int shift, float scale,
+/* Edge array and light counts the engine should use for this graph; S belongs
+ * to the caller (a plain solve or a batch). */
+static int graph_layout(adds_graph *g, Split &S, const Knobs &k, int shift, float scale,
                         const uint2 **edges, const unsigned **split) {
   if (!k.light_heavy) {
     *edges = g->edges;
     *split = nullptr;
     return ADDS_OK;
   }
-  const bool rebuild = !g->sorted_valid || !g->split_valid ||
-                       g->split_thr != light_threshold(g, shift, scale);
-  const int rc = graph_split(g, light_threshold(g, shift, scale));
+  bool rebuilt;
+  const int rc = graph_split(g, S, light_threshold(g, shift, scale), &rebuilt);
   if (rc) return rc;
   /* the rebuild ran on the graph's stream; solves may run on another */
-  if (rebuild) CK(cudaStreamSynchronize(g->stream));
+  if (rebuilt) CK(cudaStreamSynchronize(g->stream));
   *edges = g->sedges;
-  *split = g->split;
+  *split = S.at;
   return ADDS_OK;
 }
 
@@ -1409,7 +1424,7 @@ static int phase_pull_arrays(adds_graph *g, const Knobs &k, PhQuery *q) {
 static int graph_engine(adds_graph *g, const Knobs &k, int shift, float scale) {
   const uint2 *edges;
   const unsigned *split;
-  int rc = graph_layout(g, k, shift, scale, &edges, &split);
+  int rc = graph_layout(g, g->split, k, shift, scale, &edges, &split);
   if (rc) return rc;
   if (g->eng.nq == 1) {
     QueryDesc &d = g->eng.qs_host[0];
@@ -1432,7 +1447,7 @@ static int graph_engine(adds_graph *g, const Knobs &k, int shift, float scale) {
 static int graph_phase_engine(adds_graph *g, const Knobs &k, int shift, float scale) {
   const uint2 *edges;
   const unsigned *split;
-  int rc = graph_layout(g, k, shift, scale, &edges, &split);
+  int rc = graph_layout(g, g->split, k, shift, scale, &edges, &split);
   if (rc) return rc;
   PhQuery q;
   memset(&q, 0, sizeof q);
@@ -1519,8 +1534,8 @@ static float wave_delta(const adds_graph *g, int shift, float scale) {
  * R-MAT 18 0.62 both, R-MAT 16 0.49 against 0.41, all on 148 CTAs: the heavy hops
  * are extra, and fewer CTAs make edges count sooner); ER 10^6 x 8 1.0 against
  * 0.56. */
-static int wave_layout(adds_graph *g, const Knobs &k, int shift, float scale, unsigned ctas,
-                       WvQuery *q) {
+static int wave_layout(adds_graph *g, Split &S, const Knobs &k, int shift, float scale,
+                       unsigned ctas, WvQuery *q) {
   q->edges = g->edges;
   q->split = nullptr;
   q->trow = nullptr;
@@ -1528,7 +1543,7 @@ static int wave_layout(adds_graph *g, const Knobs &k, int shift, float scale, un
   if (k.wave != WV_POOL || k.light_heavy == 0 ||
       (k.light_heavy == 2 && (g->max_deg <= WV_PIECE || g->n <= 1771u * ctas)))
     return ADDS_OK;
-  int rc = graph_layout(g, k, shift, scale, &q->edges, &q->split);
+  int rc = graph_layout(g, S, k, shift, scale, &q->edges, &q->split);
   /* Heavy edges pulled where that reads less, if edges count at all: R-MAT 21 on
    * 148 CTAs 1.11 ms against 1.20, R-MAT 22 1.6 against 1.8, R-MAT 20 0.90 against
    * 0.89; 64 R-MAT 20 queries in groups of 4 18.8 against 21.2. */
@@ -1547,7 +1562,8 @@ static int graph_wave_engine(adds_graph *g, const Knobs &k, int shift, float sca
   WvQuery q;
   memset(&q, 0, sizeof q);
   q.row = g->row;
-  const int rl = wave_layout(g, k, shift, scale, k.group_ctas > 0 ? (unsigned)k.group_ctas : 148u, &q);
+  const int rl = wave_layout(g, g->split, k, shift, scale,
+                             k.group_ctas > 0 ? (unsigned)k.group_ctas : 148u, &q);
   if (rl) return rl;
   q.first = g->wfirst;
   q.piece = g->wpiece;
@@ -2013,6 +2029,7 @@ struct adds_batch {
   std::vector<uint32_t> srcs;
   std::vector<adds_graph *> ugraph; /* distinct graphs, first-use order */
   std::vector<unsigned> qgid;
+  std::vector<Split> splits; /* one per distinct graph, whose queries share a width */
   unsigned *dist_all = nullptr;
   std::vector<size_t> dist_off;
   Engine eng;
@@ -2038,7 +2055,8 @@ static int batch_phase_engine(adds_batch *b) {
     adds_graph *g = b->qgraph[i];
     const uint2 *edges;
     const unsigned *split;
-    const int rc = graph_layout(g, b->kn, b->shifts[i], b->scales[i], &edges, &split);
+    const int rc = graph_layout(g, b->splits[b->qgid[i]], b->kn, b->shifts[i], b->scales[i], &edges,
+                                &split);
     if (rc) return rc;
     PhQuery q;
     memset(&q, 0, sizeof q);
@@ -2084,7 +2102,8 @@ static int batch_wave_engine(adds_batch *b) {
     WvQuery q;
     memset(&q, 0, sizeof q);
     q.row = g->row;
-    const int rl = wave_layout(g, b->kn, b->shifts[i], b->scales[i], b->wave_group, &q);
+    const int rl = wave_layout(g, b->splits[b->qgid[i]], b->kn, b->shifts[i], b->scales[i],
+                               b->wave_group, &q);
     if (rl) return rl;
     q.first = g->wfirst;
     q.piece = g->wpiece;
@@ -2120,7 +2139,8 @@ static int batch_engine(adds_batch *b) {
     adds_graph *g = b->qgraph[i];
     const uint2 *edges;
     const unsigned *split;
-    const int rc = graph_layout(g, b->kn, b->shifts[i], b->scales[i], &edges, &split);
+    const int rc = graph_layout(g, b->splits[b->qgid[i]], b->kn, b->shifts[i], b->scales[i], &edges,
+                                &split);
     if (rc) return rc;
     qv[i] = EngQuery{g->row, edges, split, b->dist_all + b->dist_off[i], g->n, g->m, b->srcs[i],
                      b->scales[i], (unsigned)b->shifts[i], b->qgid[i]};
@@ -2195,6 +2215,7 @@ extern "C" int adds_batch_create(adds_graph *const *graphs, const uint32_t *srcs
     Knobs k;
     resolve(g, opts, &k, &b->shifts[i], &b->scales[i]);
   }
+  b->splits.resize(b->ugraph.size());
   {
     adds_opts lw;
     if (opts) lw = *opts; else adds_opts_init(&lw);
@@ -2254,6 +2275,8 @@ extern "C" void adds_batch_free(adds_batch *b) {
   engine_free(b->eng);
   ph_engine_free(b->peng);
   wv_engine_free(b->weng);
+  for (Split &s : b->splits)
+    if (s.at) cudaFree(s.at);
   if (b->dist_all) cudaFree(b->dist_all);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
@@ -2310,9 +2333,11 @@ static int batch_relayout(adds_batch *b) {
     for (size_t i = 0; i < b->qgraph.size(); ++i) {
       WvQuery &q = b->weng.qs_host[i];
       const WvQuery was = q;
-      const int rc = wave_layout(b->qgraph[i], b->kn, b->shifts[i], b->scales[i], b->wave_group, &q);
+      const int rc = wave_layout(b->qgraph[i], b->splits[b->qgid[i]], b->kn, b->shifts[i],
+                                 b->scales[i], b->wave_group, &q);
       if (rc) return rc;
-      moved = moved || q.edges != was.edges || q.split != was.split || q.trow != was.trow;
+      moved = moved || q.edges != was.edges || q.split != was.split || q.trow != was.trow ||
+              q.thr != was.thr;
     }
     for (size_t i = 0; i < b->ugraph.size(); ++i) b->wversions[i] = b->ugraph[i]->wversion;
     return moved && wv_engine_upload(b->weng, b->stream) ? ADDS_ERR_CUDA : ADDS_OK;
@@ -2320,7 +2345,8 @@ static int batch_relayout(adds_batch *b) {
   for (size_t i = 0; i < b->qgraph.size(); ++i) {
     const uint2 *edges;
     const unsigned *split;
-    const int rc = graph_layout(b->qgraph[i], b->kn, b->shifts[i], b->scales[i], &edges, &split);
+    const int rc = graph_layout(b->qgraph[i], b->splits[b->qgid[i]], b->kn, b->shifts[i],
+                                b->scales[i], &edges, &split);
     if (rc) return rc;
     if (b->kn.engine == ADDS_ENGINE_PHASE) {
       PhQuery &q = b->peng.qs_host[i];
