@@ -436,7 +436,9 @@ struct adds_graph {
   int last_shift = 0;     /* ... with this bucket shift                    */
   unsigned grow = 1;
   int tuned = 0;
-  adds_opts tuned_opts;
+  adds_opts tuned_opts; /* the fastest engine's knobs                         */
+  adds_opts tuned_wave; /* the wave kernel that beat it, as it was timed (wave
+                           0: none did)                                      */
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   Knobs last_knobs;
   EngParams last_params;
@@ -620,6 +622,7 @@ static adds_graph *graph_new(int device, adds_wtype wt) {
   g->device = device;
   g->wt = wt;
   adds_opts_init(&g->tuned_opts);
+  adds_opts_init(&g->tuned_wave);
   if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
     delete g;
@@ -1143,13 +1146,15 @@ static int auto_shift(const adds_graph *g) {
 }
 
 /* The knobs of a solve on g: the caller's, else g's tuned ones (unless
- * use_tuned is false), else the defaults. */
+ * use_tuned is false), else the defaults.  The tuned ones are an engine's: a
+ * wave kernel takes none of them. */
 static void resolve(const adds_graph *g, const adds_opts *o, Knobs *k, int *shift, float *scale,
                     bool use_tuned = true) {
   adds_opts d;
   adds_opts_init(&d);
-  const adds_opts *t = (g->tuned && use_tuned) ? &g->tuned_opts : &d;
   if (!o) o = &d;
+  const bool wave = o->wave > 0 && !g->wave_off;
+  const adds_opts *t = (g->tuned && use_tuned && !wave) ? &g->tuned_opts : &d;
   *shift = o->delta_shift >= 0 ? o->delta_shift : (t->delta_shift >= 0 ? t->delta_shift : auto_shift(g));
   *scale = o->delta_scale > 0 ? o->delta_scale : (t->delta_scale > 0 ? t->delta_scale : auto_scale(g));
   k->window = o->window > 0 ? o->window : (t->window > 0 ? t->window : 2);
@@ -1709,8 +1714,7 @@ static cudaStream_t pick_stream(const adds_graph *g, const adds_opts *o) {
  *   up to 10; R-MAT 24 4.5 against 4.2 up to 10,000, 3.6 both up to 1,000: from
  *   2^27 edges on, graphs with long rows stay with the phase engine. */
 static int auto_wave(const adds_graph *g, const adds_opts *o) {
-  if (g->wave_off || g->trace_cap || !schedule_auto(o)) return -1;
-  if (g->tuned) return g->tuned_opts.wave > 0 ? g->tuned_opts.wave - 1 : -1;
+  if (g->wave_off || g->trace_cap || g->tuned || !schedule_auto(o)) return -1;
   if (g->avg_deg < 6.0 && g->m < (1ull << 31)) return g->n < 4096u ? WV_WIDE : WV_GROUP;
   if (g->n < 32768u && g->max_deg <= WV_PIECE) return WV_GROUP; /* ER 4,001 x 8: 0.15, pooled 0.18 */
   return g->m < (g->max_deg <= WV_PIECE ? 1ull << 29 : 1ull << 27) ? WV_POOL : -1;
@@ -1744,10 +1748,17 @@ static int sssp_enqueue(adds_graph *g, uint32_t src, const adds_opts *opts) {
   int shift;
   float scale;
   Knobs k;
-  resolve(g, opts, &k, &shift, &scale);
+  adds_opts tw;
+  const adds_opts *o = opts;
+  if (g->tuned && g->tuned_wave.wave > 0 && !g->wave_off && !g->trace_cap && schedule_auto(opts)) {
+    tw = g->tuned_wave;
+    if (opts) tw.timeout_ms = opts->timeout_ms;
+    o = &tw;
+  }
+  resolve(g, o, &k, &shift, &scale);
   if (k.wave < 0) {
     k.wave = auto_wave(g, opts);
-    if (k.wave == WV_POOL && !g->tuned) shift = pooled_shift(g, shift);
+    if (k.wave == WV_POOL) shift = pooled_shift(g, shift);
   }
   if (g->wave_off) k.wave = -1;
   const bool phase = k.engine == ADDS_ENGINE_PHASE, wave = k.wave >= 0;
@@ -2707,26 +2718,33 @@ extern "C" int adds_tune(adds_graph *g, const uint32_t *srcs, uint32_t ns, adds_
     bm = descend(cur, bm, &cur);
   }
   if (bm >= 1e29) return ADDS_ERR_DEVICE_TIMEOUT;
+  /* the wave kernels, on the width that an untuned solve gives them (they adapt
+   * it); the winner is kept as it was timed, beside the engine's knobs */
+  adds_opts won;
+  adds_opts_init(&won);
   if (want == ADDS_ENGINE_AUTO && g->m < (1ull << 31)) {
-    /* the wave kernels, on the heuristic's width (they adapt it) */
-    adds_opts w;
-    adds_opts_init(&w);
-    w.engine = cur.engine;
     for (int v = 0; v <= WV_LAST; ++v) {
-      g->wave_off = false;
+      adds_opts w;
+      adds_opts_init(&w);
+      w.engine = ADDS_ENGINE_PHASE;
       w.wave = v + 1;
+      w.delta_shift = v == WV_POOL ? pooled_shift(g, auto_shift(g)) : auto_shift(g);
+      w.delta_scale = auto_scale(g);
+      g->wave_off = false;
       const double ms = time_solves(g, srcs, ns, &w);
       if (!g->wave_off && ms < bm * 0.98) { /* off: its lists overflowed */
         bm = ms;
-        cur.wave = v + 1;
+        won = w;
       }
     }
     g->wave_off = false;
+    if (won.wave == 0) wv_engine_free(g->weng); /* the lists of the last trial */
   }
   g->tuned_opts = cur;
   g->tuned_opts.stream = nullptr;
+  g->tuned_wave = won;
   g->tuned = 1;
-  if (best) *best = g->tuned_opts;
+  if (best) *best = won.wave > 0 ? won : g->tuned_opts;
   if (best_ms) *best_ms = bm / ns;
   return ADDS_OK;
 }

@@ -397,8 +397,12 @@ int adds_diag_wait_timeout(int device, int timeout_ms, double *waited_ms);
  * the phase engine the kernel variant (threads x CTAs per SM), the solo
  * threshold, the split-row threshold and the light/heavy split; for the async
  * engine window, batch, hub threshold, block, greed, CTAs/SM, order and local
- * chaining.  best may be NULL; if not, best->engine selects the engine to
- * tune on input (0 = auto) and *best receives the winner. */
+ * chaining; then, unless an engine is named, each wave kernel with the width
+ * and CTAs of an untuned solve.  If one of those wins, solves with automatic
+ * knobs run it as it was timed, and a call that sets a knob of the schedule
+ * still takes the other knobs of the fastest engine.  best may be NULL; if
+ * not, best->engine selects the engine to tune on input (0 = auto) and *best
+ * receives the winner. */
 int adds_tune(adds_graph *g, const uint32_t *srcs, uint32_t ns,
               adds_opts *best, double *best_ms);
 
