@@ -2162,7 +2162,10 @@ static int batch_engine(adds_batch *b) {
   }
   b->captured = false;
   int rc = engine_alloc(b->eng, b->device, b->flt, qv, b->grow, b->stream);
-  if (rc) return rc;
+  if (rc) {
+    engine_free(b->eng);
+    return rc;
+  }
   b->P = make_params(b->eng, b->kn, 0xFFFFFFFFu);
   return ADDS_OK;
 }
@@ -2298,7 +2301,10 @@ extern "C" void adds_batch_free(adds_batch *b) {
   delete b;
 }
 
-/* init + solve + status read-back, captured once as a CUDA graph */
+/* false between a failed layout (no memory, say) and the next launch */
+static bool batch_ready(const adds_batch *b) {
+  return (b->kn.wave >= 0 ? b->weng.nq : b->kn.engine == ADDS_ENGINE_PHASE ? b->peng.nq : b->eng.nq) != 0;
+}
 static int batch_status(const adds_batch *b) {
   if (b->kn.wave >= 0) return wv_engine_status(b->weng, g_last_err, sizeof g_last_err);
   return b->kn.engine == ADDS_ENGINE_PHASE ? phase_status(b->peng) : engine_status(b->eng);
@@ -2309,6 +2315,7 @@ static void batch_reset(adds_batch *b) {
   else engine_full_reset(b->eng, b->stream);
 }
 
+/* init + solve + status read-back, captured once as a CUDA graph */
 static int batch_capture(adds_batch *b) {
   cudaGraph_t gr = nullptr;
   CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
@@ -2381,7 +2388,7 @@ static int batch_relayout(adds_batch *b) {
 extern "C" int adds_batch_launch(adds_batch *b) {
   if (!b) return ADDS_ERR_INVALID;
   CK(cudaSetDevice(b->device));
-  const int rl = batch_relayout(b);
+  const int rl = batch_ready(b) ? batch_relayout(b) : batch_engine(b);
   if (rl) return rl;
   if (!b->captured) {
     int rc = batch_capture(b);
@@ -2393,14 +2400,32 @@ extern "C" int adds_batch_launch(adds_batch *b) {
   return ADDS_OK;
 }
 
+/* Waits for the launches in flight.  The wave kernels' lists do not grow: after
+ * an overflow the batch is laid out for its engine, from then on, and what was
+ * launched is solved there (*moved is set). */
+static int batch_wait(adds_batch *b, bool *moved) {
+  *moved = false;
+  CK(cudaStreamSynchronize(b->stream));
+  if (!batch_ready(b)) return ADDS_ERR_INVALID;
+  int rc = batch_status(b);
+  if (rc != ADDS_ERR_WL_OVERFLOW || b->kn.wave < 0) return rc;
+  *moved = true;
+  wv_engine_free(b->weng);
+  b->kn.wave = -1;
+  rc = adds_batch_launch(b);
+  if (rc) return rc;
+  CK(cudaStreamSynchronize(b->stream));
+  return batch_status(b);
+}
+
 extern "C" int adds_batch_sync(adds_batch *b, adds_stats *stats) {
   if (!b) return ADDS_ERR_INVALID;
   CK(cudaSetDevice(b->device));
-  CK(cudaStreamSynchronize(b->stream));
+  bool moved;
+  const int rc = batch_wait(b, &moved);
   const bool phase = b->kn.engine == ADDS_ENGINE_PHASE;
-  int rc = batch_status(b);
   if (rc) {
-    batch_reset(b); /* reported: the next launch starts from a clean engine */
+    if (batch_ready(b)) batch_reset(b); /* reported: the next launch starts from a clean engine */
     return rc;
   }
   if (stats) {
@@ -2420,6 +2445,7 @@ extern "C" int adds_batch_sync(adds_batch *b, adds_stats *stats) {
       stats->engine = ADDS_ENGINE_ASYNC;
     }
     stats->delta_shift = b->shifts.empty() ? 0 : b->shifts[0];
+    stats->retries = moved ? 1 : 0;
   }
   return ADDS_OK;
 }
@@ -2433,21 +2459,13 @@ extern "C" int adds_batch_run(adds_batch *b, adds_stats *stats) {
     rc = adds_batch_sync(b, stats);
     if (rc == ADDS_ERR_WL_OVERFLOW && retries < 4) {
       ++retries;
-      if (b->kn.wave >= 0) { /* its lists do not grow: the engine that does */
-        wv_engine_free(b->weng);
-        b->kn.wave = -1;
-      } else {
-        b->grow *= 2;
-      }
+      b->grow *= 2;
       rc = batch_engine(b);
       if (rc) return rc;
       continue;
     }
-    if (rc) {
-      batch_reset(b);
-      return rc;
-    }
-    if (stats) stats->retries = retries;
+    if (rc) return rc;
+    if (stats) stats->retries += retries;
     return ADDS_OK;
   }
 }
@@ -2457,8 +2475,12 @@ extern "C" int adds_batch_set_sources(adds_batch *b, const uint32_t *srcs) {
   for (size_t i = 0; i < b->srcs.size(); ++i)
     if (srcs[i] >= b->qgraph[i]->n) return ADDS_ERR_INVALID;
   CK(cudaSetDevice(b->device));
-  CK(cudaStreamSynchronize(b->stream));
+  /* a launch that overflowed is solved with the sources it had */
+  bool moved;
+  const int rw = batch_wait(b, &moved);
+  if (moved && rw) return rw;
   for (size_t i = 0; i < b->srcs.size(); ++i) b->srcs[i] = srcs[i];
+  if (!batch_ready(b)) return ADDS_OK; /* the next launch lays them out */
   if (b->kn.wave >= 0) {
     for (size_t i = 0; i < b->srcs.size(); ++i) b->weng.qs_host[i].src = srcs[i];
     return wv_engine_upload(b->weng, b->stream) ? ADDS_ERR_CUDA : ADDS_OK;

@@ -287,7 +287,9 @@ int adds_batch_create(adds_graph *const *graphs, const uint32_t *srcs,
                       uint32_t nq, const adds_opts *opts, adds_batch **out);
 int adds_batch_run(adds_batch *b, adds_stats *stats);
 /* Enqueues a run on the batch's stream without waiting; adds_batch_sync
- * waits and reports device errors. */
+ * waits and reports device errors.  If the wave kernels' lists did not suffice
+ * it solves the batch on an engine, as every later launch does
+ * (stats->retries 1). */
 int adds_batch_launch(adds_batch *b);
 int adds_batch_sync(adds_batch *b, adds_stats *stats);
 int adds_batch_dist(adds_batch *b, uint32_t q, void *dist_out);
