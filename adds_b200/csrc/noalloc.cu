@@ -200,9 +200,10 @@ __global__ void na_fill(unsigned char *B, const unsigned *row, unsigned n, unsig
  * split-row record sequence words).  Pool pages are always written before they
  * are read. */
 __global__ void na_after(unsigned char *B) {
+  if (*(const unsigned *)(B + kOffSum + 8) != 0u) return; /* na_setup set the error words */
   const unsigned err = ((const WvStat *)(B + kOffWst))->err;
   if (err != WV_ERR_OVERFLOW) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && err != WV_ERR_INPUT)
+    if (blockIdx.x == 0 && threadIdx.x == 0)
       ((PhGlobal *)(B + kOffG))->err = err == 0u ? PH_ERR_SOLVED : PH_ERR_TIMEOUT;
     return;
   }

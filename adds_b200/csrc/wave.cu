@@ -808,7 +808,7 @@ struct Wave {
     ulonglong2 *const notes =
         reinterpret_cast<ulonglong2 *>(P.grp) + ((size_t)group * 2u + par) * WV_MAX_GROUP;
     ++round;
-    const unsigned tag = round << 3; /* low bits: the error, WV_SETTLED */
+    const unsigned tag = round << WV_NOTE_BITS; /* low bits: the error, WV_SETTLED */
     ulonglong2 *const more = reinterpret_cast<ulonglong2 *>(P.grp) +
                              (size_t)P.groups * 2u * WV_MAX_GROUP +
                              ((size_t)group * 2u + par) * 2u * WV_MAX_GROUP;
@@ -833,12 +833,12 @@ struct Wave {
           const unsigned r = j * 32u + lane;
           uint4 x = make_uint4(0u, 0u, 0xFFFFFFFFu, tag);
           if (r < G) x = ld_note(notes + r);
-          here = here && (x.w & ~7u) == tag;
+          here = here && (x.w >> WV_NOTE_BITS) == (tag >> WV_NOTE_BITS);
           c[j] = x.x;
           far += x.y;
           fx = max(fx, x.y);
           fm = min(fm, x.z);
-          st |= x.w & 7u; /* two errors at once count as the worse */
+          st = wv_worse(st, x.w);
         }
         if (__all_sync(0xFFFFFFFFu, here)) break;
         late = (++it & 255u) == 0u && gtimer() > deadline;
@@ -864,7 +864,8 @@ struct Wave {
       far = __reduce_add_sync(0xFFFFFFFFu, far);
       fx = __reduce_max_sync(0xFFFFFFFFu, fx);
       fm = __reduce_min_sync(0xFFFFFFFFu, fm);
-      st = __reduce_or_sync(0xFFFFFFFFu, st);
+      st = __reduce_max_sync(0xFFFFFFFFu, st & (WV_SETTLED - 1u)) |
+           __reduce_or_sync(0xFFFFFFFFu, st & WV_SETTLED);
       /* first CTA whose entries reach into this CTA's share */
       const unsigned shr = ((tot + G - 1u) / G + 7u) & ~7u, lo = min(rank * shr, tot);
       unsigned first = 0;

@@ -9,6 +9,7 @@
 #ifndef ADDS_WAVE_INTERNAL_H_
 #define ADDS_WAVE_INTERNAL_H_
 
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 /* error word of a launch (first one wins) */
@@ -17,11 +18,20 @@
 #define WV_ERR_INPUT 3u    /* nothing to solve: the caller's arrays are invalid   */
 
 #define WV_SETTLED 4u     /* in a note: the CTA holds settled entries           */
+#define WV_NOTE_BITS 3u   /* a note's error code and WV_SETTLED                 */
 #define WV_PIECE 512u     /* edges of a long row one entry stands for          */
 #define WV_MAX_GROUP 160u /* CTAs of one group (a multiple of 32)              */
 /* a group's two sets of 16-byte notes, and (after all groups' notes) two sets
  * of 32 bytes on the settled entries */
 #define WV_GRP_WORDS (2u * (4u + 8u) * WV_MAX_GROUP)
+
+/* Two notes' states as one: the larger error code, since codes are numbers
+ * (overflow and timeout side by side are a timeout, not their OR, bad input),
+ * and whether any CTA holds settled entries. */
+static __host__ __device__ inline unsigned wv_worse(unsigned a, unsigned b) {
+  const unsigned ea = a & (WV_SETTLED - 1u), eb = b & (WV_SETTLED - 1u);
+  return (ea > eb ? ea : eb) | ((a | b) & WV_SETTLED);
+}
 
 struct WvQuery {
   const unsigned *row;
@@ -80,7 +90,6 @@ struct WvParams {
 };
 
 #ifdef __cplusplus
-#include <cuda_runtime.h>
 #include <vector>
 
 struct WvEngine {
