@@ -278,7 +278,11 @@ extern "C" int adds_sssp_noalloc(uint32_t n, uint64_t m, const uint32_t *row_sta
       area[r].ncap = kWvNcap;
       area[r].fcap = kWvFcap;
     }
-    NA_CK(cudaMemcpy((unsigned char *)p + kOffWarea, area, sizeof area, cudaMemcpyHostToDevice));
+    /* on the caller's stream, and waited for: cudaMemcpy may return before a
+     * small copy from pageable memory has arrived, and neither this call's
+     * stream nor that of a later one need wait for the default one */
+    NA_CK(cudaMemcpyAsync((unsigned char *)p + kOffWarea, area, sizeof area, cudaMemcpyHostToDevice, st));
+    NA_CK(cudaStreamSynchronize(st));
     D.base = (unsigned char *)p;
   }
   unsigned char *B = D.base;
