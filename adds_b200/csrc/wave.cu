@@ -1244,11 +1244,9 @@ int wv_engine_upload(WvEngine &E, cudaStream_t st) {
              : -5;
 }
 
-/* gsize: CTAs per query of the WV_GROUP variant (0: one per SM) */
-int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize,
-                    const std::vector<WvQuery> &qv, cudaStream_t st) {
+static int engine_layout(WvEngine &E, int device, bool flt, int shape, unsigned gsize,
+                         const std::vector<WvQuery> &qv, cudaStream_t st) {
   using namespace adds_wave;
-  wv_engine_free(E);
   E.device = device;
   E.flt = flt;
   E.shape = shape;
@@ -1349,7 +1347,6 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
     const size_t _b = (bytes_);                           \
     if (cudaMalloc((void **)&(ptr), _b) != cudaSuccess) { \
       cudaGetLastError();                                 \
-      wv_engine_free(E);                                  \
       return -4;                                          \
     }                                                     \
     E.bytes += _b;                                        \
@@ -1363,7 +1360,6 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
 #undef WV_ALLOC
   if (cudaMallocHost((void **)&E.st_host, sizeof(WvStat)) != cudaSuccess) {
     cudaGetLastError();
-    wv_engine_free(E);
     return -4;
   }
   memset(E.st_host, 0, sizeof(WvStat));
@@ -1376,6 +1372,17 @@ int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize
     return -5;
   const int rc = wv_engine_upload(E, st);
   return rc ? rc : wv_engine_reset(E, st);
+}
+
+/* gsize: CTAs per query of the group variants (0: one per SM).  E is whole
+ * afterwards or, on an error, empty: callers take an engine of the right
+ * variant and number of queries to be ready for use. */
+int wv_engine_alloc(WvEngine &E, int device, bool flt, int shape, unsigned gsize,
+                    const std::vector<WvQuery> &qv, cudaStream_t st) {
+  wv_engine_free(E);
+  const int rc = engine_layout(E, device, flt, shape, gsize, qv, st);
+  if (rc) wv_engine_free(E);
+  return rc;
 }
 
 void wv_schedule(WvParams &P, int shape) {

@@ -34,3 +34,19 @@ def test_states_of_two_notes(tmp_path, tag_a, tag_b):
                   f'  printf("%u\\n", wv_worse(a | {tag_a}u, b | {tag_b}u)); }}\n')
     want = [max(a & 3, b & 3) | ((a | b) & 4) for a in range(8) for b in range(8)]
     assert got == want
+
+
+@pytest.mark.parametrize("shape", [0, 1, 2, 3])
+def test_failed_layout_leaves_no_engine(tmp_path, shape):
+    """A device that is not there: an engine that keeps its variant and number
+    of queries without its memory would be taken for a whole one."""
+    rc, nq, shape_left, queries, pointers, size = program(
+        tmp_path, '#include "wave_internal.h"\n#include <stdio.h>\n'
+        'int main() { WvEngine E; std::vector<WvQuery> q(1, WvQuery()); q[0].n = 10; q[0].m = 20;\n'
+        f'  const int rc = wv_engine_alloc(E, -1, false, {shape}, 0, q, 0);\n'
+        '  const int held = (E.qs != 0) + (E.order != 0) + (E.area != 0) + (E.ws != 0) +\n'
+        '                   (E.st != 0) + (E.grp != 0) + (E.st_host != 0);\n'
+        '  printf("%d %u %d %zu %d %zu\\n", rc, E.nq, E.shape, E.qs_host.size(), held, E.bytes); }\n',
+        link=True)
+    assert rc == -5
+    assert (nq, shape_left, queries, pointers, size) == (0, -1, 0, 0, 0)
