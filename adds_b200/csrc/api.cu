@@ -969,7 +969,9 @@ extern "C" int adds_graph_info(const adds_graph *g, adds_graph_info_t *info) {
   info->max_degree = g->max_deg;
   info->avg_degree = g->avg_deg;
   info->avg_weight = g->avg_w;
-  info->device_bytes = g->bytes + g->eng.bytes;
+  info->device_bytes = g->bytes + g->eng.bytes + g->peng.bytes + g->weng.bytes +
+                       (g->sort_buf ? (size_t)g->m * 16 : 0) + g->sort_tmp_bytes +
+                       g->sw_cap * sizeof(SwJob);
   return ADDS_OK;
 }
 

@@ -185,7 +185,8 @@ typedef struct adds_graph_info_t {
   uint32_t max_degree;
   double avg_degree;
   double avg_weight;      /* sampled mean weight (as ads_int/kernel.cu:153-183) */
-  uint64_t device_bytes;  /* bytes held on the GPU by the graph                  */
+  uint64_t device_bytes;  /* bytes held on the GPU by the graph: its arrays, the
+                             copies and lists its solves have made so far      */
 } adds_graph_info_t;
 
 /* ---- library ------------------------------------------------------------ */
