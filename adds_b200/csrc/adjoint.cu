@@ -97,7 +97,9 @@ __global__ void k_init(const AdjQ *qs, unsigned nq) {
   }
 }
 
-/* strict tight edges: d[u] < d[v] and fl(d[u] + w) == d[v] */
+/* strict tight edges: d[u] < d[v] and fl(d[u] + w) == d[v].  Unreached vertices
+ * have none, although a weight near FLT_MAX can round to their distance word:
+ * no walk starts at them, and a parent would wait for one. */
 __global__ void k_pred_strict(const AdjQ *qs, unsigned nq) {
   ADJ_TILE(q, v0, v1)
   for (unsigned u = v0 + threadIdx.x; u < v1; u += blockDim.x) {
@@ -108,7 +110,8 @@ __global__ void k_pred_strict(const AdjQ *qs, unsigned nq) {
       const uint2 ed = q.edges[e];
       if (ed.x == q.src) continue;
       const float dv = q.dist[ed.x];
-      if (du < dv && __fadd_rn(du, __uint_as_float(ed.y)) == dv)
+      if (du < dv && __float_as_uint(dv) != ADDS_INF_F32_BITSV &&
+          __fadd_rn(du, __uint_as_float(ed.y)) == dv)
         atomicMin(&q.pred[ed.x], ((unsigned long long)e << 32) | u);
     }
   }
