@@ -425,7 +425,10 @@ struct adds_graph {
   Engine eng;
   PhEngine peng;       /* phase engine (allocated on first use)            */
   WvEngine weng;       /* wave kernels (allocated on first use)            */
-  bool wave_off = false; /* their lists overflowed on this graph           */
+  /* Their lists overflowed on this graph, or found no memory.  For good: how
+   * much is pending at once follows from its shape more than from the source
+   * or the weights, and each new try would cost the lists and a lost solve. */
+  bool wave_off = false;
   unsigned *wfirst = nullptr; /* pieces of long rows (WvQuery)              */
   uint4 *wpiece = nullptr;
   unsigned wpieces = 0;

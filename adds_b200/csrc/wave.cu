@@ -1036,7 +1036,7 @@ struct Wave {
           if (cnt == 0u) break;
           if (cnt > P.high) delta *= 0.75f;
           s_items += cnt;
-          if (POOL) hop_pool(S, w, cnt); else hop(S, w, cnt);
+          hop(S, w, cnt);
           ++hops;
           if (tid == 0 && (hops & 1023u) == 0u && gtimer() > deadline)
             S.ctr[next3(w.ci)].stop = WV_ERR_TIMEOUT;

@@ -57,7 +57,7 @@ struct WvQuery {
   unsigned long long m;
 };
 
-/* list areas of one CTA, in 16-byte entries from WvParams::ws */
+/* list areas of one CTA, in 8-byte entries from WvParams::ws */
 struct WvArea {
   unsigned long long off; /* two frontier overflow areas, then the far list    */
   unsigned ncap, fcap;    /* entries of one frontier overflow area / far list  */
