@@ -329,8 +329,8 @@ extern "C" int adds_sssp_noalloc(uint32_t n, uint64_t m, const uint32_t *row_sta
   NA_CK(cudaGetLastError());
 
   /* A wave kernel solves; where its lists do not suffice, the phase engine,
-   * which otherwise finds the solve done and returns at once (R-MAT 16: 1.33
-   * ms a call on the phase engine alone, 0.44 with the wave kernel). */
+   * which otherwise finds the solve done and returns at once (R-MAT 16: 1.27
+   * to 1.4 ms a call on the phase engine alone, 0.35 to 0.41 so, by box). */
   na_fill<<<2 * 148, 256, 0, st>>>(B, row_start, n, src, flt ? ADDS_INF_F32_BITSV : ADDS_INF_I32_BITS,
                                    dist);
   NA_CK(cudaGetLastError());

@@ -40,10 +40,12 @@
  * cycles: neighbouring entries stay together, so few of these hops relax from a
  * distance that another CTA is about to lower.
  *
- * Measured (one B200, automatic knobs, before -> now): 4096^2 road-like grid
- * 261-310 -> 18.1 ms; 517 x 301 road 16-21 -> 0.85 ms; 128 grids x 16 sources in
- * one batch 97.7 -> 7.2 ms; 60 sources on a 257 x 255 road 4.7 -> 1.6 ms; R-MAT 16
- * 0.87 -> 0.37 ms; ER 4,001 x 8 0.57 -> 0.15 ms.
+ * Measured (B200, automatic knobs, one call with its copy and wait, before ->
+ * now; the kernel alone in brackets, three graphs): 4096^2 road-like grid 261-310
+ * -> 17.9-19.9 ms (17.3-19.8); 517 x 301 road 16-21 -> 1.1-1.3 ms (0.85-1.2); 128
+ * grids x 16 sources in one batch 97.7 -> 7.2 ms; 60 sources on a 257 x 255 road 4.7
+ * -> 1.6 ms; R-MAT 16 0.87 -> 0.37-0.42 ms (0.28); ER 4,001 x 8 0.57 -> 0.16 ms
+ * (0.08-0.10).
  *
  * Graphs with long rows (POOL): rows are cut into pieces that exchanges deal
  * out, a CTA pools the edges of its entries over its threads, and on large

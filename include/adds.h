@@ -124,7 +124,9 @@ typedef struct adds_opts {
                             is automatic too), < 0 = no, 1 = a CTA of 256
                             threads, 2 = a CTA of 1024, 3 = a CTA per SM, 4 =
                             a CTA per SM that pools the edges of its entries
-                            (in a batch 3 and 4 split the SMs into groups)   */
+                            (in a batch 3 and 4 split the SMs into groups).
+                            A variant named here takes none of the knobs that
+                            adds_tune found for an engine                     */
 } adds_opts;
 
 /* Engines.  PHASE settles the buckets in bulk-synchronous phases (light
