@@ -106,3 +106,32 @@ def test_batches_of_two_widths(wtype):
     for b in bs:
         b.close()
     dg.close()
+
+
+@pytest.mark.parametrize("wtype", [G.I32, G.F32])
+def test_automatic_options(wtype):
+    """Every option automatic: the plain solve's width follows the new weights
+    and the batch's does not.  Against the phase engine on whole rows, which
+    uses no split."""
+    dg = A.Graph.generate(A.gen_spec("rmat", scale=19, wtype=wtype, w_lo=1, w_hi=10000, seed=3))
+    rng = np.random.default_rng(1)
+    srcs = [0] + [int(x) for x in rng.integers(0, dg.n, 63)]
+    b = A.Batch([dg] * 64, srcs)
+    b.run()
+    w = rng.integers(1, 301, dg.m)
+    dg.set_weights(w.astype(np.float32).view(np.uint32) if wtype == G.F32 else w.astype(np.uint32))
+    some = range(0, 64, 4)
+    want = {q: dg.sssp(srcs[q], opts(engine=PHASE, light_heavy=0))[0] for q in some}
+    for beside in (False, False, True, True, True):
+        if beside:
+            b.launch()
+            dg.sssp(5, opts(delta_shift=6, light_heavy=1))
+            dg.sssp(5)
+            b.sync()
+        else:
+            b.run()
+            dg.sssp(5)
+        for q in some:
+            assert np.array_equal(b.dist(q), want[q]), (q, beside)
+    b.close()
+    dg.close()
